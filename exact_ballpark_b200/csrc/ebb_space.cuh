@@ -1180,7 +1180,7 @@ struct World {
     EBB_HDNI bool sensor_fast(int64_t j, const double* x, const double* v, float inflated, Filing* fi) {
         int64_t a = 0, a1 = 0, ak = 0, b = 0;
         bool same = false;
-        if (!sensor_plan(j, x, v, inflated, fi, &a, &a1, &ak, &b, &same, COOP, true)) return false;
+        if (!sensor_plan(j, x, v, inflated, fi, &a, &a1, &ak, &b, &same, true)) return false;
         if (same) EBB_SENSOR_PATH(2);
         return same || sensor_count(a, a1, ak, b);
     }
@@ -1203,11 +1203,13 @@ struct World {
         return true;
     }
     // sensor_fast's conditions and counts, nothing written: a, a1, b (b = -1 when the kept count cannot move: at
-    // least 56 with room, `shortcut`), `same` when the inflated filing is the ball's own. `shared`: the scratch in
-    // the warp's shared memory (every lane on the same ball), else each thread's (or lane's) own.
+    // least 56 with room, `shortcut`), `same` when the inflated filing is the ball's own. What bounds it is its chain of
+    // dependent loads and, a lane a sensor, its divergence: with a list of the entries touched and one of the boxes made
+    // (40 and 24 entries of local memory, scanned at every step) a plan took 133,000 cycles in a 4-ship world, 4/5 of
+    // the tick there; as corner sets in registers, with the own boxes known without a lookup, the tick of 16,384
+    // 4-ship worlds a thread each takes 1.53 ms in place of 2.44.
     EBB_HDNI bool sensor_plan(int64_t j, const double* x, const double* v, float inflated, Filing* fi, int64_t* a_out,
-                              int64_t* a1_out, int64_t* ak_out, int64_t* b_out, bool* same_out, bool shared,
-                              bool shortcut) const {
+                              int64_t* a1_out, int64_t* ak_out, int64_t* b_out, bool* same_out, bool shortcut) const {
         *same_out = false;
         if (lvl(j) < 0 || huge(j) || one(s->flags) != 0) return false;
         const int64_t r = row(j);
@@ -1252,88 +1254,86 @@ struct World {
         }
         const int64_t boxi = box_find(Li, ki[0], ki[1], ki[2]);
         if (boxi < 0) return false;
-        // the boxes the ball's leaving empties: its boxes, then each parent left with nothing. The entries touched and
-        // their counts after the leaving: a warp keeps them in its shared scratch (every lane the same values), a
-        // thread in its own arrays.
-        constexpr int CAP = 40, MADE = 24;
-        int64_t own_ent[CAP], own_nb[CAP], own_nk[CAP], own_made[3 * MADE];
-        uint8_t own_gone[CAP], own_lvl[MADE];
-        int64_t *ent = own_ent, *nb = own_nb, *nk = own_nk, *made_key = own_made;
-        uint8_t *gone = own_gone, *made_lvl = own_lvl;
-#ifdef __CUDA_ARCH__
-        if (COOP && shared) {                              // (sh->key, id, out: free until GetNearbyBalls)
-            ent = sh->key;
-            nb = sh->id;
-            nk = sh->id + 64;
-            made_key = sh->key + 48;
-            gone = sh->out;
-            made_lvl = sh->out + 64;
-        }
-#endif
-        int ne = 0;
-        auto slot_of_entry = [&](int64_t e) -> int {
-            for (int i = 0; i < ne; ++i)
-                if (ent[i] == e) return i;
-            if (ne == CAP) return -1;
-            ent[ne] = e;
-            nb[ne] = BX(s->box_balls, e);
-            nk[ne] = BX(s->box_kids, e);
-            gone[ne] = 0;
-            return ne++;
+        // A filing's boxes, and their ancestors at each level above, are a product of one or two keys an axis (the
+        // ball's and its side's): a cell of them is a corner, bit q set for the side's key on axis q, bit q clear where
+        // the two keys have met at that level (`apart`: the axes still apart). So a set of such cells is 8 bits a level,
+        // in registers: no list of entries, no scan of one.
+        auto apart = [](const int64_t* k, const int64_t* m, int sh) -> unsigned {
+            unsigned on = 0;
+            for (int q = 0; q < 3; ++q)
+                if ((k[q] >> sh) != ((k[q] + m[q]) >> sh)) on |= 1u << q;
+            return on;
         };
+        // the boxes the ball's leaving empties, level by level: its own that hold it alone and no child, then each
+        // parent whose children all went and that holds no ball (`gone`: their corners, 8 bits a level)
+        const unsigned sides1 = apart(k1, m1, 0);
+        int32_t ent[8];
+        uint64_t gone = 0;
         int64_t a = 0;
-        for (int bits = 0; bits < 8; ++bits) {
-            if (((bits & 1) && !m1[0]) || ((bits & 2) && !m1[1]) || ((bits & 4) && !m1[2])) continue;
-            int64_t e = fbox(j, bits);
+        unsigned g1 = 0;
+        for (unsigned c = 0; c < 8; ++c) {
+            if (c & ~sides1) continue;
+            const int64_t e = fbox(j, (int)c);
             if (e < 0) return false;
-            int i = slot_of_entry(e);
-            if (i < 0) return false;
-            --nb[i];
-            while (nb[i] == 0 && nk[i] == 0 && !gone[i]) {
-                gone[i] = 1;
-                ++a;
-                if (BX(s->box_level, e) == 0 && e != top) return false;   // another top box emptied: its bubble lost
-                e = BX(s->box_parent, e);
-                if (e < 0) break;
-                i = slot_of_entry(e);
-                if (i < 0) return false;
-                --nk[i];
-            }
+            ent[c] = (int32_t)e;
+            if (BX(s->box_balls, e) == 1 && BX(s->box_kids, e) == 0) g1 |= 1u << c;
         }
-        // (gone: 1 released, 2 released and made again by the inflated filing's GetBox: the inflated box emptied, its
-        // chain up to a live box released and made again at once, before the sides, with the top box's bubble set)
-        auto released = [&](int64_t e) -> bool {
-            for (int i = 0; i < ne; ++i)
-                if (ent[i] == e) return gone[i] == 1;
-            return false;
+        for (int L = L1; g1 != 0; --L) {
+            gone |= (uint64_t)g1 << (8 * L);
+            if (L == 0) {
+                for (unsigned c = 0; c < 8; ++c)
+                    if ((g1 >> c) & 1) {
+                        ++a;
+                        if (ent[c] != top) return false;   // another top box emptied: its bubble lost
+                    }
+                break;
+            }
+            const unsigned keep = apart(k1, m1, 2 * (L1 - L + 1));
+            unsigned up = 0, met = 0;
+            for (unsigned c = 0; c < 8; ++c) {
+                if (!((g1 >> c) & 1)) continue;
+                ++a;
+                const unsigned q = c & keep;
+                if ((met >> q) & 1) continue;
+                met |= 1u << q;
+                int64_t kids = 0;
+                for (unsigned d = c; d < 8; ++d) kids += ((g1 >> d) & 1) && (d & keep) == q;
+                const int64_t e = BX(s->box_parent, ent[c]);
+                if (e < 0) continue;
+                ent[q] = (int32_t)e;                       // (q <= c: the corners still to come keep theirs)
+                if (BX(s->box_balls, e) == 0 && BX(s->box_kids, e) == kids) up |= 1u << q;
+            }
+            g1 = up;
+        }
+        // the corner of a cell among the own boxes and their ancestors, or 8
+        auto own_corner = [&](int L, int64_t kx, int64_t ky, int64_t kz) -> unsigned {
+            if (L > L1) return 8;
+            const int64_t k[3] = {kx, ky, kz};
+            const int sh = 2 * (L1 - L);
+            unsigned c = 0;
+            for (int q = 0; q < 3; ++q) {
+                if (k[q] == (k1[q] >> sh)) continue;
+                if (k[q] != ((k1[q] + m1[q]) >> sh)) return 8;
+                c |= 1u << q;
+            }
+            return c;
         };
-        auto gone_at = [&](int64_t e) -> int {
-            for (int i = 0; i < ne; ++i)
-                if (ent[i] == e) return i;
-            return -1;
-        };
+        int64_t a1 = 0;                                    // the ball's own box's chain
+        for (int L = L1; L >= 0 && ((gone >> (8 * L)) & 1); --L) ++a1;
+        // the inflated box emptied: its chain up to a live box made again at once by the inflated filing's GetBox, before
+        // the sides, with the top box's bubble set (`gone` keeps the boxes released and not made again)
         int64_t ak = 0;
-        for (int64_t e = boxi; e >= 0; e = BX(s->box_parent, e)) {
-            const int i = gone_at(e);
-            if (i < 0 || !gone[i]) break;
-            gone[i] = 2;
+        for (int L = Li; L >= 0; --L) {
+            const int sh = 2 * (Li - L);
+            const unsigned c = own_corner(L, ki[0] >> sh, ki[1] >> sh, ki[2] >> sh);
+            if (c == 8 || !((gone >> (8 * L + c)) & 1)) break;
+            gone &= ~(uint64_t(1) << (8 * L + c));
             ++ak;
         }
         if (ak > 0 && Li == L1) return false;             // (the ball's own box emptied, made again, emptied again)
-        int64_t a1 = 0;
-        for (int64_t e = box0; e >= 0; e = BX(s->box_parent, e)) {
-            const int i = gone_at(e);
-            if (i < 0 || !gone[i]) break;
-            ++a1;
-        }
         const int64_t g = level_grid(Li);
-        for (int side = 1; side < 8; ++side) {             // the inflated sides inside the grid
-            if (((side & 1) && !mi[0]) || ((side & 2) && !mi[1]) || ((side & 4) && !mi[2])) continue;
-            const int64_t sk[3] = {ki[0] + ((side & 1) ? mi[0] : 0), ki[1] + ((side & 2) ? mi[1] : 0),
-                                   ki[2] + ((side & 4) ? mi[2] : 0)};
-            for (int c = 0; c < 3; ++c)
-                if (sk[c] < 0 || sk[c] >= g) return false;
-        }
+        for (int c = 0; c < 3; ++c)                        // the inflated sides inside the grid
+            if (ki[c] + mi[c] < 0 || ki[c] + mi[c] >= g) return false;
         *a_out = a;
         *a1_out = a1;
         *ak_out = ak;
@@ -1343,34 +1343,31 @@ struct World {
         // at most 56 boxes made for the sides (7 chains of 8 levels): with the kept count at least that, and room for
         // them, every making takes one off it and every release puts one back (kept below 256): it ends as it began
         if (shortcut && ak == 0 && c0 >= 56 && c0 + a + 56 < BOX_KEEP && B - live >= 64) return true;
-        // else the boxes the inflated sides make, counted: each side's missing chain, up to a live box or one made
-        // before
-        int nm = 0;
+        // else the boxes the inflated sides make, counted level by level: the sides' cells that are missing, then the
+        // missing ones' parents (corner 0's chain, the inflated box's, is live). An own box or an ancestor of one is in
+        // the table, so only a cell beside them takes a lookup.
         int64_t b = 0;
-        for (int side = 1; side < 8; ++side) {
-            if (((side & 1) && !mi[0]) || ((side & 2) && !mi[1]) || ((side & 4) && !mi[2])) continue;
-            const int64_t sk[3] = {ki[0] + ((side & 1) ? mi[0] : 0), ki[1] + ((side & 2) ? mi[1] : 0),
-                                   ki[2] + ((side & 4) ? mi[2] : 0)};
-            for (int L = Li; L >= 0; --L) {
-                const int sh2 = 2 * (Li - L);
-                const int64_t kx = sk[0] >> sh2, ky = sk[1] >> sh2, kz = sk[2] >> sh2;
-                bool have = false;
-                for (int i = 0; i < nm && !have; ++i)
-                    have = made_lvl[i] == L && made_key[3 * i] == kx && made_key[3 * i + 1] == ky &&
-                           made_key[3 * i + 2] == kz;
-                if (!have) {
-                    const int64_t e = box_find(L, kx, ky, kz);
-                    have = e >= 0 && !released(e);
-                }
-                if (have) break;
-                if (nm == MADE) return false;
-                made_lvl[nm] = (uint8_t)L;
-                made_key[3 * nm] = kx;
-                made_key[3 * nm + 1] = ky;
-                made_key[3 * nm + 2] = kz;
-                ++nm;
+        unsigned want = 0;
+        const unsigned sidesi = apart(ki, mi, 0);
+        for (unsigned c = 1; c < 8; ++c)
+            if (!(c & ~sidesi)) want |= 1u << c;
+        for (int L = Li; L >= 0 && want; --L) {
+            const int sh = 2 * (Li - L);
+            const unsigned keep = L > 0 ? apart(ki, mi, sh + 2) : 0;
+            unsigned up = 0;
+            while (want) {
+                unsigned c = 0;
+                while (!((want >> c) & 1)) ++c;
+                want &= want - 1;
+                const int64_t kx = (ki[0] + ((c & 1) ? mi[0] : 0)) >> sh, ky = (ki[1] + ((c & 2) ? mi[1] : 0)) >> sh,
+                              kz = (ki[2] + ((c & 4) ? mi[2] : 0)) >> sh;
+                const unsigned o = own_corner(L, kx, ky, kz);
+                const bool have = o < 8 ? !((gone >> (8 * L + o)) & 1) : box_find(L, kx, ky, kz) >= 0;
+                if (have) continue;
                 ++b;
+                up |= 1u << (c & keep);
             }
+            want = up & ~1u;
         }
         *b_out = b;
         return true;
@@ -1541,7 +1538,7 @@ struct World {
         const double x[3] = {pos(j, 0), pos(j, 1), pos(j, 2)};
         const double v[3] = {vel(j, 0), vel(j, 1), vel(j, 2)};
         bool same = false;
-        if (!sensor_plan(j, x, v, inflated, &pr.fi, &pr.a, &pr.a1, &pr.ak, &pr.b, &same, false, false)) return;
+        if (!sensor_plan(j, x, v, inflated, &pr.fi, &pr.a, &pr.a1, &pr.ak, &pr.b, &same, false)) return;
         pr.ok = same ? 2 : 1;
         const int64_t bub = I(s->bubble, j);
         const bool excl_fixed = at(s->cloaked, j) == 0, excl_inert = at(s->sonly, j) != 0;
