@@ -8,6 +8,13 @@
 #include "../../include/ebb.h"
 #include "ebb_space.cuh"
 
+// Blocks of 4 warps a multiprocessor that the warp kernel's registers allow. A world's program is a chain of dependent
+// loads, so its length counts before the warps in flight: 128 registers (4 blocks) ran 8,000 partition worlds in 6.4 ms a
+// tick, 80 (6) in 6.6, 64 (8) in 6.7, 40 (12, with spills) in 7.2.
+#ifndef EBB_SPACE_WARP_BLOCKS
+#define EBB_SPACE_WARP_BLOCKS 4
+#endif
+
 namespace ebb {
 namespace space {
 
@@ -22,7 +29,7 @@ __global__ void __launch_bounds__(128, 6) tape_kernel(const __grid_constant__ Eb
 
 // a warp a world: the world's index is the warp's, the lanes run its program together (ebb_space.cuh's World)
 template <bool WM>
-__global__ void __launch_bounds__(128, 12) tape_kernel_warp(const __grid_constant__ EbbFlightState p,
+__global__ void __launch_bounds__(128, EBB_SPACE_WARP_BLOCKS) tape_kernel_warp(const __grid_constant__ EbbFlightState p,
                                                          const __grid_constant__ EbbSpaceState s,
                                                          const __grid_constant__ EbbSpaceTape t) {
     __shared__ Coop scratch[4];

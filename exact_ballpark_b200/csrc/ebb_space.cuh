@@ -95,12 +95,28 @@ EBB_HD int level_for(double radius) {
     return level;
 }
 
+// A sensor of a warp's batch as the scan over the slots reads it (World::scan_batch): its inflated filing's key ranges in
+// the deepest level's units, its position, bubble, range and radius; `how`: bit 0 scanned, bit 1 fixed balls left out,
+// bit 2 only interactive ones, its slot from bit 8
+struct SensorRow {
+    int64_t lo[3], hi[3];
+    double x[3];
+    int64_t bub;
+    float range, radius;
+    int32_t how, pad;
+};
+
 // A warp's scratch when a warp runs a world (EbbSpaceState.lanes = 32): the candidates' walk keys and ids by slot, and
-// their slots in the walk's order
+// their slots in the walk's order; or the rows of the batch of sensors whose candidates are being found
 struct Coop {
-    int64_t key[EBB_SPACE_MAX_SLOTS];
-    int64_t id[EBB_SPACE_MAX_SLOTS];
-    uint8_t out[EBB_SPACE_MAX_SLOTS];
+    union {
+        struct {
+            int64_t key[EBB_SPACE_MAX_SLOTS];
+            int64_t id[EBB_SPACE_MAX_SLOTS];
+            uint8_t out[EBB_SPACE_MAX_SLOTS];
+        };
+        SensorRow row[32];
+    };
 };
 
 // One world's program. A thread runs it alone (lane -1), or the 32 lanes of a warp run it together (lane 0 .. 31):
@@ -1189,17 +1205,21 @@ struct World {
     // - ak) floored (the ball's own box's chain below it made again), +b (the sides released), -(a - a1) floored (the
     // ball's own sides made again)
     EBB_HD bool sensor_count(int64_t a, int64_t a1, int64_t ak, int64_t b) {
-        const int64_t live = one(s->box_n) - one(s->box_free_n);
-        int64_t c = one(s->free_boxes);
         if (b < 0) return true;                            // (counted as unchanged: see sensor_plan)
-        if (B - live < b + ak + 8 || c + a + b >= BOX_KEEP) return false;
+        int64_t c = one(s->free_boxes);
+        if (!kept_count(c, B - (one(s->box_n) - one(s->box_free_n)), a, a1, ak, b)) return false;
+        one(s->free_boxes) = c;
+        return true;
+    }
+    // (the same on a count held by the caller; `room`: the table's free entries)
+    EBB_HD static bool kept_count(int64_t& c, int64_t room, int64_t a, int64_t a1, int64_t ak, int64_t b) {
+        if (room < b + ak + 8 || c + a + b >= BOX_KEEP) return false;
         c += a;
         c = c > ak ? c - ak : 0;
         c = c > b ? c - b : 0;
         c = c > a1 - ak ? c - (a1 - ak) : 0;
         c += b;
         c = c > a - a1 ? c - (a - a1) : 0;
-        one(s->free_boxes) = c;
         return true;
     }
     // sensor_fast's conditions and counts, nothing written: a, a1, b (b = -1 when the kept count cannot move: at
@@ -1518,22 +1538,24 @@ struct World {
 #endif
 #ifdef __CUDA_ARCH__
     // HandleProximities in a warp, 32 sensors at a time: each lane computes one sensor's check ahead (the fast path's
-    // plan, without writing, and its candidates with those in range, as slot sets), then the warp takes the map's
-    // balls in order as one ball does, using a sensor's ahead-computed check while nothing it read has changed: the
-    // world unflagged and no ball's filing changed by an earlier check's re-filings (then the rest of the batch is
-    // checked as it runs alone). The kept count moves in the map's order (sensor_count at the ball's turn).
+    // plan, without writing), the lanes together find every sensor's candidates and those in range as slot sets
+    // (scan_batch), then the warp takes the map's balls in order as one ball does, using a sensor's ahead-computed check
+    // while nothing it read has changed: the world unflagged and no ball's filing or bubble changed by an earlier check's
+    // re-filings (then the balls after it are computed ahead again). The kept count moves in the map's order. A 128-slot
+    // world's tick, in cycles: the plans 0.88 -> 0.48 million, the candidates 1.17 -> 0.36, the walk 0.92 -> 0.14, the
+    // tick's order and moved balls 0.22 -> 0.02 (8,000 partition worlds 10.2 -> 6.4 ms a tick).
     struct Pre {
         int64_t a, a1, ak, b;
         Filing fi;
         uint64_t cand[2], in[2];
         int ok;                                            // 0 none; 1 the fast path's plan; 2 and the filing the ball's own
     };
-    __device__ void pre_sensor(int64_t j, Pre& pr) const {
-        pr.ok = 0;
-        pr.cand[0] = pr.cand[1] = pr.in[0] = pr.in[1] = 0;
+    // sensor j's plan, and its row for the scan
+    __device__ void pre_sensor(int64_t j, Pre& pr, SensorRow* row_out) const {
         const int64_t r = row(j);
         const float radius = p->radius[r];
-        const float inflated = fadd(radius, (float)at(s->srange, j));
+        const float range = (float)at(s->srange, j);
+        const float inflated = fadd(radius, range);
         if (inflated < 0.0f || radius < 0.0f) return;
         const double x[3] = {pos(j, 0), pos(j, 1), pos(j, 2)};
         const double v[3] = {vel(j, 0), vel(j, 1), vel(j, 2)};
@@ -1543,25 +1565,74 @@ struct World {
         const int64_t bub = I(s->bubble, j);
         const bool excl_fixed = at(s->cloaked, j) == 0, excl_inert = at(s->sonly, j) != 0;
         if (excl_inert && !set_any(0, bub)) return;       // (no candidates)
-        const float range = (float)at(s->srange, j);
-        const int64_t S = occupied < N ? occupied : N;
-        for (int64_t o = 0; o < S; ++o) {
-            if (o == j || !slot_ok(o) || !U(s->in_park, o) || lvl(o) < 0) continue;
-            if (!related(pr.fi, o)) continue;              // (a candidate's key is made only if its membership changes)
-            const int64_t ro = row(o);
-            if (excl_inert) {
-                if (!p->interactive[ro]) continue;
-            } else {
-                if (I(s->bubble, o) != bub) continue;
-                if (excl_fixed && !p->free_[ro]) continue;
-            }
-            const uint64_t bit = uint64_t(1) << (o & 63);
-            pr.cand[o >> 6] |= bit;
-            const double ck = (double)fadd(fadd(range, p->radius[ro]), radius);
-            const double d0 = dsub(x[0], pos(o, 0)), d1 = dsub(x[1], pos(o, 1)), d2 = dsub(x[2], pos(o, 2));
-            const double len2 = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
-            if (!(len2 > dmul(ck, ck))) pr.in[o >> 6] |= bit;
+        const int sh = 2 * (NUM_LEVELS - 1 - (int)pr.fi.L);
+        for (int q = 0; q < 3; ++q) {
+            row_out->lo[q] = pr.fi.lo[q] << sh;
+            row_out->hi[q] = ((pr.fi.hi[q] + 1) << sh) - 1;
+            row_out->x[q] = x[q];
         }
+        row_out->bub = bub;
+        row_out->range = range;
+        row_out->radius = radius;
+        row_out->how = 1 | (excl_fixed ? 2 : 0) | (excl_inert ? 4 : 0) | ((int32_t)j << 8);
+    }
+    // The batch's candidates and those in range: a lane a slot, its filing, position and filters in registers, against
+    // every sensor of the batch (its row a broadcast from shared memory); two ballots a sensor are its sets' words.
+    // A lane a sensor instead, walking the slots, spent 4,100 cycles a slot on the slot's dependent loads (three
+    // quarters of the check's time in a 128-slot world). Relatedness (related): in the deepest level's units a key
+    // range is the interval of the cells it covers, and the finer range shifted up meets the coarser's exactly when
+    // the intervals meet.
+    __device__ void scan_batch(Pre& mine, unsigned sensors) const {
+        uint32_t cw[4] = {0, 0, 0, 0}, iw[4] = {0, 0, 0, 0};
+        const int S = occupied < N ? occupied : (int)N;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (32 * q >= S) break;
+            const int64_t o = 32 * q + lane;
+            bool ok = o < S && slot_ok(o) && U(s->in_park, o) && lvl(o) >= 0;
+            int64_t lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0}, bub = 0;
+            double x[3] = {0.0, 0.0, 0.0};
+            float radius = 0.0f;
+            bool free_o = false, inter = false;
+            if (ok) {
+                const Filing f = filing_of(o);
+                const int sh = 2 * (NUM_LEVELS - 1 - (int)f.L);
+                const int64_t ro = row(o);
+                for (int c = 0; c < 3; ++c) {
+                    lo[c] = f.lo[c] << sh;
+                    hi[c] = ((f.hi[c] + 1) << sh) - 1;
+                    x[c] = pos(o, c);
+                }
+                bub = I(s->bubble, o);
+                radius = p->radius[ro];
+                free_o = p->free_[ro] != 0;
+                inter = p->interactive[ro] != 0;
+            }
+            for (unsigned left = sensors; left; left &= left - 1) {
+                const int i = __ffs(left) - 1;
+                const SensorRow& t = sh->row[i];
+                const int how = t.how;
+                bool c = ok && (how >> 8) != (int)o && ((how & 4) ? inter : (t.bub == bub && (free_o || !(how & 2))));
+                c = c && t.lo[0] <= hi[0] && lo[0] <= t.hi[0] && t.lo[1] <= hi[1] && lo[1] <= t.hi[1] &&
+                    t.lo[2] <= hi[2] && lo[2] <= t.hi[2];
+                const unsigned cb = __ballot_sync(0xffffffffu, c);
+                unsigned ib = 0;
+                if (cb) {
+                    const double ck = (double)fadd(fadd(t.range, radius), t.radius);
+                    const double d0 = dsub(t.x[0], x[0]), d1 = dsub(t.x[1], x[1]), d2 = dsub(t.x[2], x[2]);
+                    const double len2 = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
+                    ib = __ballot_sync(0xffffffffu, c && !(len2 > dmul(ck, ck)));
+                }
+                if (lane == i) {
+                    cw[q] = cb;
+                    iw[q] = ib;
+                }
+            }
+        }
+        mine.cand[0] = (uint64_t)cw[0] | ((uint64_t)cw[1] << 32);
+        mine.cand[1] = (uint64_t)cw[2] | ((uint64_t)cw[3] << 32);
+        mine.in[0] = (uint64_t)iw[0] | ((uint64_t)iw[1] << 32);
+        mine.in[1] = (uint64_t)iw[2] | ((uint64_t)iw[3] << 32);
     }
     __device__ static Pre pre_of(const Pre& mine, int i) {
         Pre o;
@@ -1643,12 +1714,12 @@ struct World {
         __syncwarp();
     }
     // CheckSensor at the ball's turn with its ahead-computed check (else as it runs alone; `dirty` when that
-    // changed the ball's filing)
+    // changed the ball's filing or bubble)
     __device__ void check_sensor_pre(int64_t j, const Pre& pr, bool& dirty) {
         at(s->selapsed, j) = dadd(at(s->selapsed, j), p->dt);
         if (at(s->selapsed, j) < at(s->speriod, j)) return;
         at(s->selapsed, j) = 0.0;
-        if (pr.ok && !dirty && one(s->flags) == 0 && (pr.ok == 2 || sensor_count(pr.a, pr.a1, pr.ak, pr.b))) {
+        if (pr.ok && one(s->flags) == 0 && (pr.ok == 2 || sensor_count(pr.a, pr.a1, pr.ak, pr.b))) {
             EBB_SENSOR_PATH(0);
             EBB_SENSOR_PATH(1);
             if (pr.ok == 2) EBB_SENSOR_PATH(2);
@@ -1656,29 +1727,106 @@ struct World {
             return;
         }
         const int64_t l0 = lvl(j), k0 = key(j, 0), k1 = key(j, 1), k2 = key(j, 2), m0 = mod(j, 0), m1 = mod(j, 1),
-                      m2 = mod(j, 2), a0 = active(j);
+                      m2 = mod(j, 2), a0 = active(j), b0 = I(s->bubble, j);
         check_sensor_body(j);
         if (lvl(j) != l0 || key(j, 0) != k0 || key(j, 1) != k1 || key(j, 2) != k2 || mod(j, 0) != m0 ||
-            mod(j, 1) != m1 || mod(j, 2) != m2 || active(j) != a0)
+            mod(j, 1) != m1 || mod(j, 2) != m2 || active(j) != a0 || I(s->bubble, j) != b0)
             dirty = true;
     }
-    __device__ void handle_proximities_warp(const uint8_t* keys, int32_t n) {
-        for (int32_t batch = 0; batch < n; batch += 32) {
+    // The proximity balls in the map's order, its entries 32 q + lane in this lane's byte q of `keys`. Most checks change
+    // nothing but the elapsed time and the kept count ("quiet": no notification range or tracking, the sensor's period
+    // come or not, the ahead-computed sets equal to its list): the lanes find those at once, and the warp's walk over
+    // the order only moves the kept count by each (its four terms packed in a word, at most 64 each); the others are
+    // taken whole at their turn.
+    __device__ void handle_proximities_warp(uint32_t keys, int32_t n) {
+        int32_t batch = 0;
+        while (batch < n) {
             Pre mine;
             mine.ok = 0;
             mine.a = mine.a1 = mine.ak = mine.b = 0;
             mine.fi = Filing{};
-            mine.cand[0] = mine.cand[1] = mine.in[0] = mine.in[1] = 0;
-            if (batch + lane < n) {
-                const int64_t j = keys[batch + lane];
-                if (slot_ok(j) && U(s->in_park, j) && p->sensor[row(j)]) pre_sensor(j, mine);
+            const int e_mine = batch + lane;
+            int64_t j_mine = -1;
+            {
+                const uint32_t k = __shfl_sync(0xffffffffu, keys, e_mine & 31);   // (a batch may start anywhere)
+                if (e_mine < n) j_mine = (k >> (8 * (e_mine >> 5))) & 255;
             }
+            sh->row[lane].how = 0;
+            const bool live = j_mine >= 0 && slot_ok(j_mine) && U(s->in_park, j_mine);
+            const bool senses = live && p->sensor[row(j_mine)];
+            if (senses) pre_sensor(j_mine, mine, &sh->row[lane]);
             __syncwarp();
+            scan_batch(mine, __ballot_sync(0xffffffffu, sh->row[lane].how & 1));
+            // 0: taken whole at its turn; 1: not due; 2: due, no event
+            int quiet = 0;
+            double elapsed = 0.0;
+            if (senses && at(s->has_prox, j_mine) && at(s->ntf_range, j_mine) == 0.0 &&
+                !(at(s->trk_range, j_mine) >= TRACKING_MIN && at(s->trk, j_mine) >= 0) && !in_dead_bubble(j_mine)) {
+                elapsed = dadd(at(s->selapsed, j_mine), p->dt);
+                if (elapsed < at(s->speriod, j_mine)) {
+                    quiet = 1;
+                } else if (mine.ok) {
+                    elapsed = 0.0;
+                    const UMap m = sensor_map(j_mine);
+                    const uint64_t m0 = m.m[0], m1 = m.m[m.mstep];
+                    const uint64_t self0 = j_mine < 64 ? uint64_t(1) << j_mine : 0,
+                                   self1 = j_mine < 64 ? 0 : uint64_t(1) << (j_mine - 64);
+                    if (((m0 & ~mine.cand[0] & ~self0) | (m1 & ~mine.cand[1] & ~self1) |
+                         (mine.cand[0] & (mine.in[0] ^ m0)) | (mine.cand[1] & (mine.in[1] ^ m1))) == 0)
+                        quiet = 2;
+                }
+            }
+            const unsigned not_due = __ballot_sync(0xffffffffu, quiet == 1), calm = __ballot_sync(0xffffffffu, quiet == 2),
+                           same = __ballot_sync(0xffffffffu, mine.ok == 2);
+            const uint32_t terms = (uint32_t)mine.a | ((uint32_t)mine.a1 << 8) | ((uint32_t)mine.ak << 16) |
+                                   ((uint32_t)(mine.b & 255) << 24);
+            __syncwarp();
+            unsigned taken = 0;                            // the quiet ones passed at their turn
             bool dirty = false;
             const int32_t end = n < batch + 32 ? n : batch + 32;
-            for (int32_t e = batch; e < end; ++e) {
+            int32_t e = batch;
+            while (e < end && !dirty) {
+                // a run of quiet balls, the kept count in a register
+                const int i0 = e - batch;
+                if (((not_due | calm) >> i0) & 1) {
+                    const bool unflagged = one(s->flags) == 0;
+                    const int64_t room = B - (one(s->box_n) - one(s->box_free_n));
+                    const int64_t c0 = one(s->free_boxes);
+                    int64_t c = c0;
+                    bool stop = false;
+                    while (e < end && !stop) {
+                        const int i = e - batch;
+                        if ((not_due >> i) & 1) {
+                            taken |= 1u << i;
+                            ++e;
+                            continue;
+                        }
+                        if (!((calm >> i) & 1)) break;
+                        if (!unflagged) {
+                            stop = true;
+                            break;
+                        }
+                        if (!((same >> i) & 1)) {
+                            const uint32_t t = __shfl_sync(0xffffffffu, terms, i);
+                            const int64_t a = t & 255, a1 = (t >> 8) & 255, ak = (t >> 16) & 255, b = t >> 24;
+                            if (!kept_count(c, room, a, a1, ak, b)) {
+                                stop = true;
+                                break;
+                            }
+                        } else {
+                            EBB_SENSOR_PATH(2);
+                        }
+                        EBB_SENSOR_PATH(0);
+                        EBB_SENSOR_PATH(1);
+                        taken |= 1u << i;
+                        ++e;
+                    }
+                    if (c != c0) one(s->free_boxes) = c;
+                    if (!stop) continue;
+                }
                 const Pre pr = pre_of(mine, e - batch);
-                const int64_t j = keys[e];
+                const int64_t j = __shfl_sync(0xffffffffu, j_mine, e - batch);
+                ++e;
                 if (!slot_ok(j) || !U(s->in_park, j)) continue;
                 if (in_dead_bubble(j)) {
                     if (at(s->slen, j) > 0) {
@@ -1695,6 +1843,9 @@ struct World {
                 check_target_tracking(j);
                 if (p->sensor[row(j)]) check_sensor_pre(j, pr, dirty);
             }
+            if ((taken >> lane) & 1) at(s->selapsed, j_mine) = elapsed;
+            __syncwarp();
+            batch = e;
         }
     }
 #endif
@@ -1708,27 +1859,31 @@ struct World {
     EBB_HDNI void handle_proximities() {
         const UMap pm = proximity_map();
         const int32_t n = *pm.len;
-        uint8_t keys[EBB_SPACE_MAX_SLOTS];
-        for (int32_t e = 0; e < n; ++e) keys[e] = pm.k[e * pm.step];
 #ifdef __CUDA_ARCH__
         if constexpr (COOP) {
+            uint32_t keys = 0;
+            for (int q = 0; q < 4; ++q)
+                if (32 * q + lane < n) keys |= (uint32_t)pm.k[(32 * q + lane) * pm.step] << (8 * q);
             handle_proximities_warp(keys, n);
-            return;
-        }
+        } else
 #endif
-        for (int32_t e = 0; e < n; ++e) {
-            const int64_t j = keys[e];
-            if (!slot_ok(j) || !U(s->in_park, j)) continue;
-            if (in_dead_bubble(j)) {
-                if (at(s->slen, j) > 0) {
-                    at(s->selapsed, j) = at(s->speriod, j);
-                    check_for_proximity(j);
+        {
+            uint8_t keys[EBB_SPACE_MAX_SLOTS];
+            for (int32_t e = 0; e < n; ++e) keys[e] = pm.k[e * pm.step];
+            for (int32_t e = 0; e < n; ++e) {
+                const int64_t j = keys[e];
+                if (!slot_ok(j) || !U(s->in_park, j)) continue;
+                if (in_dead_bubble(j)) {
+                    if (at(s->slen, j) > 0) {
+                        at(s->selapsed, j) = at(s->speriod, j);
+                        check_for_proximity(j);
+                    }
+                    umap_clear(sensor_map(j));
+                    continue;
                 }
-                umap_clear(sensor_map(j));
-                continue;
+                if (!at(s->has_prox, j)) continue;
+                check_for_proximity(j);
             }
-            if (!at(s->has_prox, j)) continue;
-            check_for_proximity(j);
         }
     }
 
@@ -1935,38 +2090,26 @@ struct World {
         one(s->dict_n) = m;
     }
     // phase 1's dead-bubble flags: a free ball of the park in a dead bubble skips the tick
-    EBB_HD void dead() {
-        for (int64_t j = 0; j < N; ++j) {
+    EBB_HD void dead() {                                   // (in a warp a lane a slot)
+        for (int64_t j = COOP ? lane : 0; j < N; j += COOP ? 32 : 1) {
             const bool in = U(s->in_park, j) && slot_ok(j);
             U(s->dead, j) = (in && p->free_[row(j)] && in_dead_bubble(j)) ? 1 : 0;
         }
+#ifdef __CUDA_ARCH__
+        if constexpr (COOP) __syncwarp();
+#endif
     }
     // after the park's tick, in ascending id: each warp drop-out nearly at rest re-filed at its drop-out point (the old
     // state), then each ball that moved at least sqrt(0.1) m
     EBB_HDNI void after_evolve() {
-        int64_t order[EBB_SPACE_MAX_SLOTS];
-        int64_t n = 0;
 #ifdef __CUDA_ARCH__
-        if constexpr (COOP) {                              // the lanes sort the slots by id together
-            int mine = 0, last = -1;
-            const int S = sort_span();
-            for (int64_t j = lane; j < S; j += 32) {
-                const bool in = j < N && U(s->in_park, j) && slot_ok(j);
-                sh->key[j] = in ? 0 : NOT_A_CANDIDATE;
-                sh->id[j] = in ? id(j) : INT64_MAX;
-                sh->out[j] = (uint8_t)j;
-                mine += in;
-                if (in) last = (int)j;
-            }
-            n = (int64_t)__reduce_add_sync(0xffffffffu, (unsigned)mine);
-            occupied = (int)__reduce_max_sync(0xffffffffu, (unsigned)(last + 1));
-            __syncwarp();
-            warp_sort(S);
-            for (int64_t i = 0; i < n; ++i) order[i] = sh->out[i];
-            __syncwarp();
+        if constexpr (COOP) {
+            after_evolve_warp();
         } else
 #endif
         {
+            int64_t order[EBB_SPACE_MAX_SLOTS];
+            int64_t n = 0;
             for (int64_t j = 0; j < N; ++j)
                 if (U(s->in_park, j) && slot_ok(j)) order[n++] = j;
             for (int64_t i = 1; i < n; ++i)
@@ -1975,49 +2118,92 @@ struct World {
                     order[k] = order[k - 1];
                     order[k - 1] = t;
                 }
-        }
-        for (int64_t i = 0; i < n; ++i) {
-            const int64_t j = order[i], r = row(j);
-            if (!U(s->dropped, j) || U(s->dead, j) || !p->free_[r]) continue;
-            const double ov[3] = {p->old_vel[r], p->old_vel[p->n + r], p->old_vel[2 * p->n + r]};
-            if (!(dadd(dadd(dmul(ov[0], ov[0]), dmul(ov[1], ov[1])), dmul(ov[2], ov[2])) < 0.1)) continue;
-            const double op[3] = {p->old_pos[r], p->old_pos[p->n + r], p->old_pos[2 * p->n + r]};
-            insert_in_boxes(j, op, ov);
-        }
-        // the commits' re-filings; a warp first finds, a lane a ball, those whose re-filing leaves everything as it is
-        // (refile_noop: nothing an earlier ball's re-filing writes changes that), and files the others in id order
-        uint64_t noop[2] = {0, 0};
-#ifdef __CUDA_ARCH__
-        if constexpr (COOP) {
-            for (int64_t i0 = 0; i0 < n; i0 += 32) {
-                bool q = false;
-                int64_t jj = -1;
-                if (i0 + lane < n) {
-                    jj = order[i0 + lane];
-                    q = !U(s->dead, jj) && p->free_[row(jj)] && refile_noop(jj);
-                }
-                unsigned bits = __ballot_sync(0xffffffffu, q);
-                while (bits) {
-                    const int b = __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    const int64_t k = __shfl_sync(0xffffffffu, jj, b);
-                    noop[k >> 6] |= uint64_t(1) << (k & 63);
-                }
-            }
-        }
-#endif
-        for (int64_t i = 0; i < n; ++i) {
-            const int64_t j = order[i], r = row(j);
-            if (U(s->dead, j) || !p->free_[r]) continue;
-            double d[3];
-            for (int c = 0; c < 3; ++c) d[c] = dsub(p->pos[c * p->n + r], p->old_pos[c * p->n + r]);
-            if (!(dadd(dadd(dmul(d[0], d[0]), dmul(d[1], d[1])), dmul(d[2], d[2])) < 0.1)) {
-                if (!((noop[j >> 6] >> (j & 63)) & 1)) insert_in_boxes(j);
+            for (int64_t i = 0; i < n; ++i)
+                if (drops_out(order[i])) refile_dropped(order[i]);
+            for (int64_t i = 0; i < n; ++i) {
+                const int64_t j = order[i];
+                if (!moved(j)) continue;
+                insert_in_boxes(j);
                 set_fresh(j, true);
             }
         }
         handle_proximities();
     }
+    // a warp's drop-out nearly at rest; a ball of the tick that moved
+    EBB_HD bool drops_out(int64_t j) const {
+        const int64_t r = row(j);
+        if (!U(s->dropped, j) || U(s->dead, j) || !p->free_[r]) return false;
+        const double ov[3] = {p->old_vel[r], p->old_vel[p->n + r], p->old_vel[2 * p->n + r]};
+        return dadd(dadd(dmul(ov[0], ov[0]), dmul(ov[1], ov[1])), dmul(ov[2], ov[2])) < 0.1;
+    }
+    EBB_HD void refile_dropped(int64_t j) {
+        const int64_t r = row(j);
+        const double ov[3] = {p->old_vel[r], p->old_vel[p->n + r], p->old_vel[2 * p->n + r]};
+        const double op[3] = {p->old_pos[r], p->old_pos[p->n + r], p->old_pos[2 * p->n + r]};
+        insert_in_boxes(j, op, ov);
+    }
+    EBB_HD bool moved(int64_t j) const {
+        const int64_t r = row(j);
+        if (U(s->dead, j) || !p->free_[r]) return false;
+        double d[3];
+        for (int c = 0; c < 3; ++c) d[c] = dsub(p->pos[c * p->n + r], p->old_pos[c * p->n + r]);
+        return !(dadd(dadd(dmul(d[0], d[0]), dmul(d[1], d[1])), dmul(d[2], d[2])) < 0.1);
+    }
+#ifdef __CUDA_ARCH__
+    // after_evolve in a warp: the order, the drop-outs and the balls that moved are found a lane a ball, with those
+    // whose re-filing leaves everything as it is (refile_noop: nothing an earlier ball's re-filing writes changes
+    // that); the warp files the others one after another in id order
+    __device__ void after_evolve_warp() {
+        int n = 0, last = -1;
+        for (int64_t base = 0; base < N; base += 32) {     // the slots in the park, packed in slot order
+            const int64_t j = base + lane;
+            const bool in = j < N && U(s->in_park, j) && slot_ok(j);
+            const unsigned bits = __ballot_sync(0xffffffffu, in);
+            if (in) {
+                const int e = n + __popc(bits & ((1u << lane) - 1u));
+                sh->key[e] = 0;
+                sh->id[e] = id(j);
+                sh->out[e] = (uint8_t)j;
+            }
+            n += __popc(bits);
+            if (bits) last = (int)base + 31 - __clz(bits);
+        }
+        occupied = last + 1;
+        __syncwarp();
+        bool rising = true;                                // (a world added in id order needs no sort)
+        for (int e = lane; e + 1 < n; e += 32) rising = rising && sh->id[e] < sh->id[e + 1];
+        if (!__all_sync(0xffffffffu, rising)) {
+            int P = 1;
+            while (P < n) P <<= 1;
+            for (int e = n + lane; e < P; e += 32) {
+                sh->key[e] = NOT_A_CANDIDATE;
+                sh->id[e] = INT64_MAX;
+            }
+            __syncwarp();
+            warp_sort(P);
+        }
+        uint32_t order = 0;                                // entry 32 q + lane in byte q
+        for (int q = 0; q < 4; ++q)
+            if (32 * q + lane < n) order |= (uint32_t)sh->out[32 * q + lane] << (8 * q);
+        __syncwarp();
+        for (int q = 0; 32 * q < n; ++q) {
+            const int64_t j = (order >> (8 * q)) & 255;
+            unsigned bits = __ballot_sync(0xffffffffu, 32 * q + lane < n && drops_out(j));
+            for (; bits; bits &= bits - 1) refile_dropped(__shfl_sync(0xffffffffu, j, __ffs(bits) - 1));
+        }
+        for (int q = 0; 32 * q < n; ++q) {
+            const int64_t j = (order >> (8 * q)) & 255;
+            const bool on = 32 * q + lane < n && moved(j);
+            unsigned bits = __ballot_sync(0xffffffffu, on && !refile_noop(j));
+            for (; bits; bits &= bits - 1) insert_in_boxes(__shfl_sync(0xffffffffu, j, __ffs(bits) - 1));
+            uint32_t f[4];
+            for (int c = 0; c < 4; ++c)
+                f[c] = __reduce_or_sync(0xffffffffu, on && (int)(j >> 5) == c ? 1u << (j & 31) : 0u);
+            fresh[0] |= (uint64_t)f[0] | ((uint64_t)f[1] << 32);
+            fresh[1] |= (uint64_t)f[2] | ((uint64_t)f[3] << 32);
+        }
+    }
+#endif
     // Whether InsertInBoxes of ball j at its position and velocity changes nothing: the same box (level and keys) with
     // its entries kept, its top's bubble the ball's, the same sides. Read-only; for the tick's re-filings.
     EBB_HD bool refile_noop(int64_t j) const {
