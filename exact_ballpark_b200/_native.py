@@ -18,6 +18,7 @@ ABI = 8
 COLLIDE_MAX_SLOTS = 64          # include/ebb.h: EBB_COLLIDE_MAX_SLOTS
 COLLIDE_MAX_STATICS = 64        # include/ebb.h: EBB_COLLIDE_MAX_STATICS
 SPACE_MAX_SLOTS = 128           # include/ebb.h: EBB_SPACE_MAX_SLOTS
+SPACE_MAX_LAYERS = 8
 RAND_WORDS = 33                 # include/ebb.h: EBB_RAND_WORDS
 
 _lib = None
@@ -142,6 +143,8 @@ def lib() -> ctypes.CDLL:
                                   p, i32]
     L.ebb_space_tape.argtypes = [ctypes.POINTER(FlightState), ctypes.POINTER(SpaceState), ctypes.POINTER(SpaceTape), p,
                                  i32]
+    L.ebb_space_tapes.argtypes = [ctypes.POINTER(FlightState), ctypes.POINTER(SpaceState), ctypes.POINTER(SpaceTape), i32,
+                                  p]
     L.ebb_glibc_srand.argtypes = [p, i64, p, p]
     L.ebb_glibc_rand.argtypes = [p, i64, i64, p, p]
     L.ebb_flight_snap.argtypes = [ctypes.POINTER(FlightState), p, i32, p, i32]

@@ -25,11 +25,11 @@ import numpy as np
 import torch
 
 from .modes import WARP, VecModesPark
-from .space import OP, VecSpace
+from .space import OP, VecSpace, tick_op
 
 CLASSES = (4, 8, 16, 32, 64, 128)
 WARP_CLASS = 32                  # the ragged batch's classes from this size up run a warp a world
-BOOL, I64 = torch.bool, torch.int64
+BOOL, I64, U8 = torch.bool, torch.int64, torch.uint8
 
 
 class PartitionLayer:
@@ -97,11 +97,12 @@ class PartitionLayer:
     # ---- the tick ----
     def dead_rows(self) -> torch.Tensor:
         """Every layer's dead-bubble rows [n] (phase 1's flags)."""
-        dead = None
-        for layer, _ in self.layers:
-            d = layer.dead_rows()
-            dead = d if dead is None else dead | d
-        return dead
+        layers = [layer for layer, _ in self.layers]
+        tick_op(layers, "DEAD")
+        dead = torch.zeros(self.park.n + 1, dtype=BOOL, device=self.park.dev)
+        for layer in layers:                             # (their rows are apart; a slot without a row has the last entry)
+            layer.scatter_dead(dead)
+        return dead[:self.park.n]
 
     def tick(self, park_tick=None) -> None:
         """One tick of the park with the layer: the dead bubbles' balls left out of the park's tick (flagged
@@ -119,9 +120,11 @@ class PartitionLayer:
             park_tick()
         park._moribund.copy_(saved)
         dropped = warp_proper & (park._mode != WARP)
+        padded = torch.cat([dropped.to(U8), torch.zeros(1, dtype=U8, device=park.dev)])
         for layer, _ in self.layers:
             layer.clear_events()
-            layer.after_evolve(dropped)
+            layer.gather_dropped(padded)
+        tick_op([layer for layer, _ in self.layers], "AFTER_EVOLVE")
 
     # ---- readers ----
     def event_counts(self) -> torch.Tensor:

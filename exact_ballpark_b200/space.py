@@ -118,6 +118,24 @@ def allocate_state(spec, W: int, dev, world_major: bool):
     return out, pitch
 
 
+def tick_op(layers: list, name: str) -> None:
+    """A tick's operation (DEAD or AFTER_EVOLVE) on every world of `layers`, layers over one park that share no row of
+    it: those that run a warp a world over the world-major state in one launch (ebb_space_tapes), the ones of most
+    slots first (the longest programs start first), each other layer in a launch of its own."""
+    warp = sorted((x for x in layers if x.lanes == 32 and x.pitch > 0), key=lambda x: -x.N)
+    for k in range(0, len(warp), _native.SPACE_MAX_LAYERS):
+        some = warp[k:k + _native.SPACE_MAX_LAYERS]
+        park = some[0].park
+        states = (_native.SpaceState * len(some))(*(x.state() for x in some))
+        tapes = (_native.SpaceTape * len(some))(*(_native.SpaceTape(1, *(t.data_ptr() for t in x._tick_ops[name]), None)
+                                                  for x in some))
+        rc = _native.lib().ebb_space_tapes(ctypes.byref(park.state()), states, tapes, len(some), park._stream())
+        _native.check(rc, "ebb_space_tapes")
+    for x in layers:
+        if x.lanes != 32 or not x.pitch:
+            x.broadcast(name)
+
+
 class VecSpace:
     """The layer for W worlds of N slots over a flight park's rows. `rows` [W, N]: the park's row of each slot (-1 for
     none), each world's slots in the order its balls are added. Capacities a world: `boxes` box-table entries,
@@ -166,6 +184,8 @@ class VecSpace:
         self._flat = torch.where(self.rows >= 0, self.rows, park.n).t().flatten()   # [W N] slot -> row, n for none
         self._state = None
         self.last_dead = None
+        self._tick_ops = {name: tuple(torch.full((W,), v, dtype=I64, device=d) for v in (OP[name], -1, 0))
+                          for name in ("DEAD", "AFTER_EVOLVE")}    # the tick's operations on every world, made once
 
     # ---- plumbing ----
 
@@ -261,18 +281,25 @@ class VecSpace:
         """Phase 1's dead-bubble flags [n] (TIME-714) for the park's tick to skip, no host synchronisation."""
         self.broadcast("DEAD", worlds)
         out = torch.zeros(self.park.n + 1, dtype=BOOL, device=self.dev)
-        out.scatter_(0, self._flat, self.st["dead"].t().flatten().to(BOOL))
+        self.scatter_dead(out)
         return out[:self.park.n]
+
+    def scatter_dead(self, out: torch.Tensor) -> None:
+        """The layer's dead-bubble flags at its rows of `out` [n + 1] (the last entry a slot without a row)."""
+        out.scatter_(0, self._flat, self.st["dead"].t().flatten().to(BOOL))
 
     def after_evolve(self, dropped_rows: torch.Tensor | None = None, worlds: torch.Tensor | None = None) -> None:
         """After the park's tick: the warp drop-outs' re-filings, then the commits' (no host synchronisation)."""
-        dr = self.st["dropped"]
         if dropped_rows is None:
-            dr.zero_()
+            self.st["dropped"].zero_()
         else:
-            pad = torch.cat([dropped_rows.to(self.dev).to(U8), torch.zeros(1, dtype=U8, device=self.dev)])
-            dr.copy_(pad[self._flat].reshape(self.W, self.N).t())
+            self.gather_dropped(torch.cat([dropped_rows.to(self.dev).to(U8),
+                                           torch.zeros(1, dtype=U8, device=self.dev)]))
         self.broadcast("AFTER_EVOLVE", worlds)
+
+    def gather_dropped(self, padded: torch.Tensor) -> None:
+        """The layer's rows of the drop-outs' flags `padded` [n + 1] (uint8, the last entry 0)."""
+        self.st["dropped"].copy_(padded[self._flat].reshape(self.W, self.N).t())
 
     def tick(self) -> None:
         """One tick of the park with the layer, as Destiny's Evolve runs it on the master: the dead bubbles' balls left

@@ -425,6 +425,12 @@ int ebb_libm(int func, int64_t n, const double* x, const double* y, double* out,
  * (exact_ballpark/vec_space.py:896). */
 int ebb_space_tape(const EbbFlightState* park, const EbbSpaceState* s, const EbbSpaceTape* t, void* stream, int block);
 
+/* The same for `count` layers over one park (at most EBB_SPACE_MAX_LAYERS), layer l's tape t[l] on its state s[l], in one
+ * launch: their worlds run beside one another, those of the first layer first. Every layer a warp a world over the
+ * world-major arrangement, and no two sharing a row of the park. No counterpart in the reference. */
+#define EBB_SPACE_MAX_LAYERS 8
+int ebb_space_tapes(const EbbFlightState* park, const EbbSpaceState* s, const EbbSpaceTape* t, int count, void* stream);
+
 /* One query a world (EbbSpaceQuery), one thread a world, on `stream`; nothing but the answer written. Replaces
  * xbps_query_cuda (exact_ballpark/vec_space.py:938). */
 int ebb_space_query(const EbbFlightState* park, const EbbSpaceState* s, const EbbSpaceQuery* q, void* stream,

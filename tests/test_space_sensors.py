@@ -51,3 +51,34 @@ def test_batches_of_sensors_on_the_device(lanes, ships, spread):
     import torch
     assert torch.cuda.is_available()
     assert not _differ(ships, spread, 4, lambda ops, seed: sl.drive_ticks(ops, seed=seed, lanes=lanes))
+
+
+def test_several_layers_tapes_refuse_bad_arguments_before_launching():
+    """ebb_space_tapes: too many layers, a thread-a-world or interleaved layer among them, a missing buffer; nothing to
+    do without layers, worlds or operations."""
+    import ctypes
+
+    from exact_ballpark_b200 import _native
+    lib = _native.lib()
+    p = _native.FlightState()
+    s, t = (_native.SpaceState * 2)(), (_native.SpaceTape * 2)()
+    call = lambda n=2: lib.ebb_space_tapes(ctypes.byref(p), s, t, n, None)  # noqa: E731
+    for k in range(2):
+        for st in (p, s[k], t[k]):
+            for name, kind in type(st)._fields_:
+                if kind is ctypes.c_void_p:
+                    setattr(st, name, 4096)
+        s[k].worlds, s[k].slots, s[k].boxes, s[k].dicts, s[k].entries, s[k].sets = 0, 10, 64, 16, 16, 16
+        s[k].umap_cap, s[k].events, s[k].lanes, s[k].pitch, t[k].K = 10, 16, 32, 1024, 1
+    assert call(0) == 0 and call() == 0                   # no layers; no worlds
+    assert call(-1) == -1 and call(_native.SPACE_MAX_LAYERS + 1) == -1
+    s[1].worlds = 4
+    for name, wrong in (("lanes", 1), ("pitch", 0), ("slots", 129), ("fbox", None), ("lanes", 7)):
+        keep = getattr(s[1], name)
+        setattr(s[1], name, wrong)
+        assert call() == -1, name
+        setattr(s[1], name, keep)
+    t[1].code = None
+    assert call() == -1
+    t[1].K = 0
+    assert call() == 0                                    # no operations
