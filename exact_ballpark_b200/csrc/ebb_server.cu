@@ -1,5 +1,5 @@
 // SPDX-License-Identifier: MIT
-// The server layer over the flight park on the device, one thread a world (include/ebb.h: ebb_server_tick). What
+// The server layer over the flight park on the device, one lane or a few a world (include/ebb.h: ebb_server_tick). What
 // exact_ballpark.vec_server.VecServer's torch path does for a tick's queue (vec_server.py:707-1060) in one launch:
 //
 //   stamps    each world's stamp for its calls and the next one (the world's park time + 1);
@@ -17,7 +17,7 @@
 //             uncloak's AddBallsToPark recipients marked;
 //   flags     after the park's tick: per row, whether its pilot gets the bubble's narrowcast and a character update.
 //
-// A world's calls are sequential, so its thread walks them in order; worlds never touch each other's rows. Each
+// A world's calls are sequential where they touch (Group below); worlds never touch each other's rows. Each
 // command is stated for one row in the order of operations the torch path's row-parallel version uses, with the
 // rounding pinned as in the flight tick (doubles by __dadd_rn and friends, the setters' float arguments rounded to
 // float, the rotation in float).
@@ -42,27 +42,12 @@ struct World {
     const int64_t* rows;                                  // the world's rows, -1 padded to s.width
     const int64_t* ids;
 
-    __device__ int64_t lookup(int64_t id) const {        // the first listed ball with this id (a pad's id is 0)
-        return lookup(id, s.width);
-    }
-    // the same over the first `span` positions, past which the world has pads alone (row -1: the same answer)
+    // the first listed ball with this id (a pad's id is 0) over the first `span` positions, past which the world has pads
+    // alone (row -1: the same answer)
     __device__ int64_t lookup(int64_t id, int64_t span) const {
         for (int64_t k = 0; k < span; ++k)
             if (ids[k] == id) return rows[k];
         return -1;
-    }
-    __device__ int64_t listed_span() const {              // one past the world's last listed ball
-        int64_t span = 0;
-        for (int64_t k = 0; k < s.width; ++k)
-            if (rows[k] >= 0) span = k + 1;
-        return span;
-    }
-    __device__ bool any_interactive() const {
-        for (int64_t k = 0; k < s.width; ++k) {
-            const int64_t r = rows[k];
-            if (r >= 0 && p.interactive[r] && s.exists[r]) return true;
-        }
-        return false;
     }
 
     // ---- Stop(Ball*) and the commands that move a ball (vec_modes.py:289-420) ----
@@ -297,11 +282,57 @@ struct World {
     }
 };
 
-// The queue pass: each push's rows, CloakBall's bubble and the duplicate test, nothing written to the park (so the
-// loads of later slots need not wait for earlier slots' commands); the world's ids held in registers for the lookups.
+// ---- a group of G lanes a world ----
+//
+// A world's queue is G slots at a time, a lane a slot; its rows a lane a row. What a thread a world did one after another
+// in a chain of dependent loads (8 slots and 4 rows: 39 us for 65,536 worlds at 18 % of DRAM's peak; 256 slots and 128
+// rows: 1.17 ms for 8,000 worlds, 63 blocks) the group's lanes do at once, except where a call's effect reaches another's:
+// - the duplicate test compares a call with the last queued one. A duplicate equals what it repeats, so comparing with
+//   the last call pushed before it, queued or not, gives the same answer: no chain, that slot read again;
+// - calls on one row apply in queue order by that row's first lane of the chunk; a call writes its own ball's row alone and
+//   reads no other's, but for EntityWarpIn (its followers), and FollowBall or Orbit (the target's cloak, which
+//   UncloakBall writes): a queue with those is walked by one lane;
+// - a queued CloakBall (its followers, and the routes after it) has the history walked by one lane.
+// The lanes of a warp's groups stay together (the loops' counts are the batch's), so the votes are the warp's.
+template <int G>
+struct Group {
+    int lane, sub, first;                                 // the lane, its place in the group, the group's first lane
+    bool on;                                              // the group has a world
+    unsigned mask;                                        // its lanes
+    __device__ explicit Group(bool has_world) {
+        lane = threadIdx.x & 31;
+        sub = lane & (G - 1);
+        first = lane & ~(G - 1);
+        on = has_world;
+        mask = (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << first);
+    }
+    __device__ bool any(bool v) const {
+        if constexpr (G == 1) return v;
+        return (__ballot_sync(0xffffffffu, v) & mask) != 0;
+    }
+    __device__ bool all(bool v) const { return !any(!v); }
+    // the highest lane of the group below this one with the flag, and of the whole group, -1 for none
+    __device__ int before(bool v) const {
+        const unsigned m = __ballot_sync(0xffffffffu, v) & mask & ((1u << lane) - 1u);
+        return m ? 31 - __clz(m) : -1;
+    }
+    __device__ int last(bool v) const {
+        const unsigned m = __ballot_sync(0xffffffffu, v) & mask;
+        return m ? 31 - __clz(m) : -1;
+    }
+};
+
+// CloakBall's bubble or a call's own local flag, as the duplicate test compares it (a tested call's is given)
+__device__ int64_t loc_of(const EbbServerState& s, int32_t kind, bool tested, int64_t row, int64_t loc_in) {
+    return !tested && kind == EBB_KIND_CLOAK ? (s.settled[row < 0 ? 0 : row] ? 0 : -1) : loc_in;
+}
+
+// The queue pass by a world's only lane (worlds of at most IDS_IN_REGISTERS rows): each push's rows, CloakBall's bubble and
+// the duplicate test, nothing written to the park (so the loads of later slots need not wait for earlier slots'
+// commands); the world's ids held in registers for the lookups.
 constexpr int IDS_IN_REGISTERS = 8;
 
-__device__ void queue(const World& x, const EbbServerQueue& q) {
+__device__ void queue_alone(const World& x, const EbbServerQueue& q) {
     const EbbServerState& s = x.s;
     const int64_t W = s.worlds, w = x.w, J = q.slots;
     const int32_t* __restrict__ kinds = q.kinds;
@@ -321,14 +352,7 @@ __device__ void queue(const World& x, const EbbServerQueue& q) {
         ids[k] = k < s.width ? x.ids[k] : 0;
         rows[k] = k < s.width ? x.rows[k] : -1;
     }
-    const int64_t span = s.width > IDS_IN_REGISTERS ? x.listed_span() : s.width;
-    // a wide world whose listed balls are ids 1, 2, ... in order (each id once, no pad among them): a ball's row is
-    // then at its id's position, and an id outside them is no ball's (the pads past them have row -1)
-    bool ordered = s.width > IDS_IN_REGISTERS;
-    for (int64_t k = 0; ordered && k < span; ++k) ordered = x.ids[k] == k + 1 && x.rows[k] >= 0;
     auto lookup = [&](int64_t id) -> int64_t {
-        if (ordered) return id >= 1 && id <= span ? x.rows[id - 1] : -1;
-        if (s.width > IDS_IN_REGISTERS) return x.lookup(id, span);
         int64_t found = -1;
 #pragma unroll
         for (int k = IDS_IN_REGISTERS - 1; k >= 0; --k)       // the first match wins
@@ -379,30 +403,149 @@ __device__ void queue(const World& x, const EbbServerQueue& q) {
     }
 }
 
-__device__ void queue_and_apply(const World& x, const EbbServerQueue& q) {
+// Whether the world's listed balls are ids 1, 2, ... in order up to its last (a ball's row is then at its id's position,
+// and an id outside them is no ball's), and one past the last listed
+template <int G>
+__device__ bool ids_in_order(const World& x, const Group<G>& g, int64_t* span_out) {
+    int64_t span = 0;
+    bool ordered = true;
+    for (int64_t k0 = 0; k0 < x.s.width; k0 += G) {
+        const int64_t k = k0 + g.sub;
+        const bool listed = g.on && k < x.s.width && x.rows[k] >= 0;
+        const bool fits = !g.on || k >= x.s.width || (listed ? x.ids[k] == k + 1 : true);
+        const unsigned m = __ballot_sync(0xffffffffu, listed) & g.mask;
+        if (m) {
+            // the positions up to this chunk's last listed ball all listed, and the chunk follows the one before
+            const int at = 31 - __clz(m);
+            const unsigned want = g.mask & ((2u << at) - 1u);
+            if (m != want || span != k0) ordered = false;
+            span = k0 + (at - g.first) + 1;
+        }
+        ordered = g.all(fits) && ordered;
+    }
+    *span_out = span;
+    return ordered;
+}
+
+// The queue pass: each push's rows, CloakBall's bubble and the duplicate test; nothing written to the park. Returns whether
+// the queue must be applied by one lane.
+template <int G>
+__device__ bool queue(const World& x, const EbbServerQueue& q, const Group<G>& g) {
+    const EbbServerState& s = x.s;
+    const int64_t W = s.worlds, w = x.w, J = q.slots;
+    int64_t span;
+    const bool ordered = ids_in_order(x, g, &span);
+    auto lookup = [&](int64_t id) -> int64_t {
+        if (ordered) return id >= 1 && id <= span ? x.rows[id - 1] : -1;
+        return x.lookup(id, span);
+    };
+    int64_t last = -1;                                    // the slot of the world's last pushed call (none yet: all zero)
+    bool warps_in = false, follows = false, uncloaks = false;
+    for (int64_t j0 = 0; j0 < J; j0 += G) {
+        const int64_t j = j0 + g.sub;
+        const bool here = g.on && j < J;
+        const int64_t a = j * W + w;
+        int32_t kind = 0;
+        int64_t ball = 0, target = 0, n = 0, loc = 0, row = -1, trow = -1;
+        double f[4] = {0.0, 0.0, 0.0, 0.0};
+        bool pushed = false, tested = false;
+        if (here) {
+            kind = q.kinds[j];
+            ball = q.ball[a];
+            target = q.target[a];
+            n = q.n[a];
+            for (int k = 0; k < 4; ++k) f[k] = q.f[a * 4 + k];
+            const uint8_t byte = q.mask[a];
+            row = lookup(ball);
+            if (kind == EBB_KIND_FOLLOW_BALL || kind == EBB_KIND_ORBIT) trow = lookup(target);
+            tested = (byte & 2) != 0;                     // tested already by an undo: bit 0 is its queued flag
+            loc = loc_of(s, kind, tested, row, q.loc_in[a]);
+            pushed = (byte & 1) != 0 && (tested || kind != EBB_KIND_CLOAK || row >= 0);
+        }
+        const int near = g.before(pushed);
+        const int64_t p = near < 0 ? last : j0 + (near - g.first);
+        bool same = false;
+        if (pushed && !tested) {
+            if (p < 0) {
+                same = kind == 0 && ball == 0 && target == 0 && f[0] == 0.0 && f[1] == 0.0 && f[2] == 0.0 &&
+                       f[3] == 0.0 && n == 0 && loc == 0;
+            } else if (q.kinds[p] == kind) {
+                const int64_t b = p * W + w;
+                same = q.ball[b] == ball && q.target[b] == target && q.n[b] == n;
+                for (int k = 0; k < 4; ++k) same = same && q.f[b * 4 + k] == f[k];
+                if (same)                                 // (the same ball: the same row)
+                    same = loc_of(s, kind, (q.mask[b] & 2) != 0, row, q.loc_in[b]) == loc;
+            }
+        }
+        const bool ok = pushed && !same;
+        const int end = g.last(pushed);
+        if (end >= 0) last = j0 + (end - g.first);
+        if (here) {
+            q.ok[a] = ok;
+            q.row[a] = row;
+            q.trow[a] = trow;
+            q.loc[a] = loc;
+        }
+        const bool acts = ok && row >= 0;
+        warps_in = warps_in || (acts && kind == EBB_KIND_ENTITY_WARP_IN);
+        follows = follows || (acts && (kind == EBB_KIND_FOLLOW_BALL || kind == EBB_KIND_ORBIT));
+        uncloaks = uncloaks || (acts && kind == EBB_KIND_UNCLOAK);
+    }
+    const bool wi = g.any(warps_in), fo = g.any(follows), un = g.any(uncloaks);
+    __syncwarp();
+    return wi || (fo && un);
+}
+
+// one queued call applied (every one but CloakBall)
+__device__ void apply_slot(const World& x, const EbbServerQueue& q, int64_t j) {
+    const int64_t a = j * x.s.worlds + x.w;
+    const int32_t kind = q.kinds[j];
+    const int64_t row = q.row[a];
+    if (!q.ok[a] || row < 0 || kind == EBB_KIND_CLOAK) return;
+    const double f[4] = {q.f[a * 4], q.f[a * 4 + 1], q.f[a * 4 + 2], q.f[a * 4 + 3]};
+    x.apply(kind, row, q.trow[a], f, q.n[a]);
+}
+
+template <int G>
+__device__ void queue_and_apply(const World& x, const EbbServerQueue& q, const Group<G>& g) {
     const EbbServerState& s = x.s;
     const int64_t W = s.worlds, w = x.w;
-    const int64_t clock = x.p.clock[x.rows[0]];
-    q.clock[w] = clock;
-    q.stamp[w] = s.stamp_for_system[w];
-    s.stamp_for_system[w] = clock + 1;
-    queue(x, q);
-    for (int64_t j = 0; j < q.slots; ++j) {               // every queued call but CloakBall, in queue order
-        const int64_t a = j * W + w;
-        const int32_t kind = q.kinds[j];
-        const int64_t row = q.row[a];
-        if (!q.ok[a] || row < 0 || kind == EBB_KIND_CLOAK) continue;
-        const double f[4] = {q.f[a * 4], q.f[a * 4 + 1], q.f[a * 4 + 2], q.f[a * 4 + 3]};
-        x.apply(kind, row, q.trow[a], f, q.n[a]);
+    const int64_t clock = g.on ? x.p.clock[x.rows[0]] : 0;
+    if (g.on && g.sub == 0) {
+        q.clock[w] = clock;
+        q.stamp[w] = s.stamp_for_system[w];
+        s.stamp_for_system[w] = clock + 1;
     }
+    bool serial = true;                                   // (a world's only lane walks its queue)
+    if constexpr (G == 1) {
+        if (g.on) queue_alone(x, q);
+    } else {
+        serial = queue(x, q, g);
+    }
+    for (int64_t j0 = 0; G > 1 && j0 < q.slots; j0 += G) {         // every queued call but CloakBall, each row's in queue order
+        const int64_t j = j0 + g.sub;
+        long long row = -1 - g.lane;                      // (a lane without a call is alone)
+        if (g.on && !serial && j < q.slots) {
+            const int64_t a = j * W + w;
+            if (q.ok[a] && q.row[a] >= 0) row = q.row[a];
+        }
+        unsigned calls = __match_any_sync(0xffffffffu, row);
+        if (row >= 0 && g.lane == __ffs(calls) - 1)
+            for (; calls; calls &= calls - 1) apply_slot(x, q, j0 + (__ffs(calls) - 1 - g.first));
+        __syncwarp();
+    }
+    if (g.on && serial && g.sub == 0)
+        for (int64_t j = 0; j < q.slots; ++j) apply_slot(x, q, j);
+    __syncwarp();
     // the bubble update, once per park time
-    if (clock == s.bubble_time[w]) return;
-    bool any_listed = false;
-    for (int64_t k = 0; k < s.width; ++k) {
+    const bool due = g.on && clock != s.bubble_time[w];
+    bool listed_here = false;
+    for (int64_t k = g.sub; due && k < s.width; k += G) {
         const int64_t r = x.rows[k];
-        if (r >= 0 && s.exists[r] && s.cloaked[r] == 0) any_listed = true;
+        if (r >= 0 && s.exists[r] && s.cloaked[r] == 0) listed_here = true;
     }
-    for (int64_t k = 0; k < s.width; ++k) {
+    const bool any_listed = g.any(listed_here);
+    for (int64_t k = g.sub; due && k < s.width; k += G) {
         const int64_t r = x.rows[k];
         if (r < 0) continue;
         const bool user = x.p.interactive[r] && s.exists[r];
@@ -410,69 +553,84 @@ __device__ void queue_and_apply(const World& x, const EbbServerQueue& q) {
         s.listed[r] = s.exists[r] && s.cloaked[r] == 0;
         if (user) s.settled[r] = 1;
     }
-    s.bubble_time[w] = clock;
+    __syncwarp();
+    if (due && g.sub == 0) s.bubble_time[w] = clock;
 }
 
-__device__ void history(const World& x, const EbbServerQueue& q, int64_t j0, int64_t j1) {
-    const EbbServerState& s = x.s;
-    const int64_t W = s.worlds, w = x.w, R = x.p.n;
-    const bool live = x.any_interactive();
-    for (int64_t j = j0; j < j1; ++j) {
-        const int64_t a = j * W + w;
-        const int32_t kind = q.kinds[j];
-        const bool ok = q.ok[a] != 0;
-        const int64_t row = q.row[a];
-        const bool valid = ok && row >= 0;
-        int8_t route = EBB_ROUTE_NONE;
-        if (kind == EBB_KIND_CLOAK) {
-            if (ok && q.loc[a] == 0) route = EBB_ROUTE_BUBBLE;
-            if (valid) x.cloak(row, q.n[a], q.f[a * 4]);
-        } else if (kind == EBB_KIND_UNCLOAK) {
-            if (valid && live && x.p.interactive[row] && s.pilot[row] >= 0) route = EBB_ROUTE_CHARACTER;
-            for (int64_t k = 0; k < s.width; ++k) {
-                const int64_t r = x.rows[k];
-                if (r < 0) continue;
-                q.notice[j * R + r] = valid && live && x.p.interactive[r] && s.exists[r] && r != row && s.pilot[r] >= 0;
-            }
-        } else {
-            const bool go = (kind == EBB_KIND_SET_POSITION) ? (valid && q.loc[a] == 0 && live)
-                                                             : (valid && live && q.ball[a] > 0);
-            if (go) route = x.route_of(row);
-        }
-        q.route[j * s.worlds + w] = route;
+template <int G>
+__device__ bool any_interactive(const World& x, const Group<G>& g) {
+    bool here = false;
+    for (int64_t k = g.sub; g.on && !here && k < x.s.width; k += G) {
+        const int64_t r = x.rows[k];
+        here = r >= 0 && x.p.interactive[r] && x.s.exists[r];
     }
+    return g.any(here);
 }
 
-__device__ void flags(const World& x, const EbbServerQueue& q) {
+// one slot of the history (CloakBall applied there)
+__device__ void history_slot(const World& x, const EbbServerQueue& q, int64_t j, bool live) {
+    const EbbServerState& s = x.s;
+    const int64_t a = j * s.worlds + x.w, R = x.p.n;
+    const int32_t kind = q.kinds[j];
+    const bool ok = q.ok[a] != 0;
+    const int64_t row = q.row[a];
+    const bool valid = ok && row >= 0;
+    int8_t route = EBB_ROUTE_NONE;
+    if (kind == EBB_KIND_CLOAK) {
+        if (ok && q.loc[a] == 0) route = EBB_ROUTE_BUBBLE;
+        if (valid) x.cloak(row, q.n[a], q.f[a * 4]);
+    } else if (kind == EBB_KIND_UNCLOAK) {
+        if (valid && live && x.p.interactive[row] && s.pilot[row] >= 0) route = EBB_ROUTE_CHARACTER;
+        for (int64_t k = 0; k < s.width; ++k) {
+            const int64_t r = x.rows[k];
+            if (r < 0) continue;
+            q.notice[j * R + r] = valid && live && x.p.interactive[r] && s.exists[r] && r != row && s.pilot[r] >= 0;
+        }
+    } else {
+        const bool go = (kind == EBB_KIND_SET_POSITION) ? (valid && q.loc[a] == 0 && live)
+                                                         : (valid && live && q.ball[a] > 0);
+        if (go) route = x.route_of(row);
+    }
+    q.route[a] = route;
+}
+
+template <int G>
+__device__ void history(const World& x, const EbbServerQueue& q, const Group<G>& g, int64_t j0, int64_t j1) {
+    const bool live = any_interactive(x, g);
+    bool cloaks = false;
+    for (int64_t j = j0 + g.sub; g.on && j < j1; j += G) {
+        const int64_t a = j * x.s.worlds + x.w;
+        cloaks = cloaks || (q.kinds[j] == EBB_KIND_CLOAK && q.ok[a] && q.row[a] >= 0);
+    }
+    const bool serial = g.any(cloaks);
+    if (g.on && !serial)
+        for (int64_t j = j0 + g.sub; j < j1; j += G) history_slot(x, q, j, live);
+    if (g.on && serial && g.sub == 0)
+        for (int64_t j = j0; j < j1; ++j) history_slot(x, q, j, live);
+    __syncwarp();
+}
+
+template <int G>
+__device__ void flags(const World& x, const EbbServerQueue& q, const Group<G>& g) {
     const EbbServerState& s = x.s;
     const int64_t W = s.worlds, w = x.w, R = x.p.n, J = q.slots;
-    bool bubble = false;
-    uint64_t character[2] = {0, 0};                       // the world's rows (by position) routed to their character
-    bool uncloaks = false;
-    for (int64_t j = 0; j < J; ++j) {
+    bool bubble_here = false, character_here = false, uncloaks = false;
+    for (int64_t j = g.sub; g.on && j < J; j += G) {
         const int8_t route = q.route[j * W + w];
-        bubble = bubble || route == EBB_ROUTE_BUBBLE;
+        bubble_here = bubble_here || route == EBB_ROUTE_BUBBLE;
+        character_here = character_here || (route == EBB_ROUTE_CHARACTER && q.ok[j * W + w]);
         uncloaks = uncloaks || q.kinds[j] == EBB_KIND_UNCLOAK;
-        if (route != EBB_ROUTE_CHARACTER) continue;
-        const int64_t a = j * W + w;
-        if (!q.ok[a]) continue;
-        const int64_t row = q.row[a];
-        for (int64_t k = 0; k < s.width && k < 128; ++k)
-            if (x.rows[k] == row) character[k >> 6] |= uint64_t(1) << (k & 63);
     }
-    for (int64_t k = 0; k < s.width; ++k) {
+    const bool bubble = g.any(bubble_here), character = g.any(character_here), any_uncloak = g.any(uncloaks);
+    for (int64_t k = g.sub; g.on && k < s.width; k += G) {
         const int64_t r = x.rows[k];
         if (r < 0) continue;
         bool has = s.fresh[r] != 0;
-        if (k < 128) {
-            has = has || ((character[k >> 6] >> (k & 63)) & 1u);
-        } else {                                          // a world wider than the mask: the slots again
-            for (int64_t j = 0; j < J && !has; ++j) {
-                const int64_t a = j * W + w;
-                has = q.ok[a] && q.row[a] == r && q.route[j * W + w] == EBB_ROUTE_CHARACTER;
-            }
+        for (int64_t j = 0; j < J && character && !has; ++j) {   // (the world has a call routed to a character)
+            const int64_t a = j * W + w;
+            has = q.route[a] == EBB_ROUTE_CHARACTER && q.ok[a] && q.row[a] == r;
         }
-        for (int64_t j = 0; j < J && uncloaks && !has; ++j)
+        for (int64_t j = 0; j < J && any_uncloak && !has; ++j)
             has = q.kinds[j] == EBB_KIND_UNCLOAK && q.notice[j * R + r];
         const bool pilot = s.pilot[r] >= 0;
         q.has_character[r] = has && pilot;
@@ -480,33 +638,59 @@ __device__ void flags(const World& x, const EbbServerQueue& q) {
     }
 }
 
-__global__ void __launch_bounds__(128) server_kernel(EbbServerState s, EbbServerQueue q, int phase, int64_t j0,
+// (4 blocks a multiprocessor, 128 registers: latency-bound; a lane a world of 65,536 takes 24.7 us so, 30.7 us at 5 blocks,
+// 40.1 at 6)
+template <int G>
+__global__ void __launch_bounds__(128, 4) server_kernel(const __grid_constant__ EbbServerState s,
+                                                      const __grid_constant__ EbbServerQueue q, int phase, int64_t j0,
                                                       int64_t j1) {
-    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= s.worlds) return;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const Group<G> g(w < s.worlds);
     const World x{s, s.flight, w, s.world_rows + w * s.width, s.world_ids + w * s.width};
     switch (phase) {
         case 0:
-            queue_and_apply(x, q);
-            history(x, q, 0, q.slots);
+        case 5:                                           // 5: phase 0, then the park's tick's dead-bubble test
+            queue_and_apply(x, q, g);
+            history(x, q, g, 0, q.slots);
             break;
-        case 1: queue_and_apply(x, q); break;
-        case 2: history(x, q, j0, j1); break;
-        case 3: flags(x, q); break;
-        case 4:
-            if (!x.any_interactive()) s.dead[w] = 1;
+        case 1: queue_and_apply(x, q, g); break;
+        case 2: history(x, q, g, j0, j1); break;
+        case 3: flags(x, q, g); break;
+        case 6:                                           // the queue's test alone: flags, rows, CloakBall's bubble
+            if constexpr (G == 1) {
+                if (g.on) queue_alone(x, q);
+            } else {
+                queue(x, q, g);
+            }
             break;
-        case 5:                                           // phase 0, then the park's tick's dead-bubble test
-            queue_and_apply(x, q);
-            history(x, q, 0, q.slots);
-            if (!x.any_interactive()) s.dead[w] = 1;
-            break;
-        case 6: queue(x, q); break;                       // the queue's test alone: flags, rows, CloakBall's bubble
         default: break;
+    }
+    if (phase == 4 || phase == 5) {
+        const bool live = any_interactive(x, g);
+        if (g.on && g.sub == 0 && !live) s.dead[w] = 1;
     }
 }
 
-cudaError_t attributes(cudaFuncAttributes* fa) { return cudaFuncGetAttributes(fa, server_kernel); }
+// The lanes a world, from its queue's slots and its rows, the `most` of the two. One when there are worlds enough to keep
+// the chip's warps in flight a thread each (a thread's accesses then coalesce with its neighbours', and nothing is voted
+// on); else enough for the slots and rows at once, up to a warp (a larger queue or world is taken 32 at a time). Pre-tick
+// and flags of 4-ship worlds (8 slots), us, one lane and eight: 8,192 worlds 22.9 and 15.9; 16,384 21.9 and 21.5; 24,576
+// 24.2 and 23.6; 32,768 25.7 and 31.2; 65,536 30.4 and 56.2. One ship (2 slots), 24,576 worlds: 9.8 and 20.5 (four lanes,
+// 65,536 worlds: 11.3 and 33.9). 8,000 worlds of 1 to 128 ships (256 slots): 1,436 us and, a warp a world, 140.
+enum class Lanes { one, four, eight, half, warp };
+inline Lanes lanes(int64_t worlds, int64_t most) {
+    if (most <= IDS_IN_REGISTERS && worlds > 2048 * most) return Lanes::one;
+    return most <= 4 ? Lanes::four : most <= 8 ? Lanes::eight : most <= 16 ? Lanes::half : Lanes::warp;
+}
+template <int G>
+cudaError_t launch(const EbbServerState& s, const EbbServerQueue& q, int phase, int64_t j0, int64_t j1, cudaStream_t st,
+                   int block) {
+    const unsigned grid = (unsigned)((s.worlds + block / G - 1) / (block / G));
+    server_kernel<G><<<grid, block, 0, st>>>(s, q, phase, j0, j1);
+    return cudaGetLastError();
+}
+
+cudaError_t attributes(cudaFuncAttributes* fa) { return cudaFuncGetAttributes(fa, server_kernel<8>); }
 
 }  // namespace server
 }  // namespace ebb
@@ -533,9 +717,13 @@ int ebb_server_tick(const EbbServerState* s, const EbbServerQueue* q, int phase,
          q->loc_in == nullptr || q->f == nullptr || q->ok == nullptr || q->row == nullptr || q->trow == nullptr ||
          q->loc == nullptr || q->route == nullptr || q->notice == nullptr))
         return EBB_EINVAL;
-    const unsigned grid = (unsigned)((s->worlds + block - 1) / block);
-    ebb::server::server_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(*s, *q, phase, j0, j1);
-    const cudaError_t e = cudaGetLastError();
+    const cudaStream_t st = (cudaStream_t)stream;
+    const ebb::server::Lanes g = ebb::server::lanes(s->worlds, q->slots > s->width ? q->slots : s->width);
+    const cudaError_t e = g == ebb::server::Lanes::one     ? ebb::server::launch<1>(*s, *q, phase, j0, j1, st, block)
+                          : g == ebb::server::Lanes::four  ? ebb::server::launch<4>(*s, *q, phase, j0, j1, st, block)
+                          : g == ebb::server::Lanes::eight ? ebb::server::launch<8>(*s, *q, phase, j0, j1, st, block)
+                          : g == ebb::server::Lanes::half  ? ebb::server::launch<16>(*s, *q, phase, j0, j1, st, block)
+                                                           : ebb::server::launch<32>(*s, *q, phase, j0, j1, st, block);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
