@@ -86,7 +86,7 @@ struct Rec {
 
 __host__ __device__ inline size_t records_bytes(int block) { return ((size_t)block * sizeof(Rec) + 15) & ~(size_t)15; }
 __host__ __device__ inline size_t smem_bytes(int block) {
-    return records_bytes(block) + (size_t)(block / 32) * KTAB_FLOATS * sizeof(float);
+    return records_bytes(block) + (size_t)(block / 32) * ORIENT_FLOATS * sizeof(float);
 }
 
 // StopAllFollowers on this follower (vec_combat_cuda.cu:216; MOV-730): a missile is made non-massive and, like an
@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(256, COLLIDE ? EBB_COMPOSED_MIN_BLOCKS : EBB_C
         return;
     }
     Rec* rec = (Rec*)smem_raw;
-    float* ktab = (float*)(smem_raw + records_bytes(blockDim.x)) + (threadIdx.x >> 5) * KTAB_FLOATS;
+    float* found = (float*)(smem_raw + records_bytes(blockDim.x)) + (threadIdx.x >> 5) * ORIENT_FLOATS;
     fill_ndt(ndt_tab, c.flight.dt);
     const int m = (int)(r1 - r0);
     const int j = threadIdx.x;
@@ -968,7 +968,7 @@ __global__ void __launch_bounds__(256, COLLIDE ? EBB_COMPOSED_MIN_BLOCKS : EBB_C
         if (COLLIDE && c.flight.free_[i] && !c.flight.moribund[i]) clear_contacts(x, i);
         phase1(c, i, r0, r1, rec, d, &release_after, status);
     }
-    orient_warp(d, cfg_of(c.flight), ndt_tab, ktab);
+    orient_warp(d, cfg_of(c.flight), ndt_tab, found);
     if (mine) phase1_end(c, i, d, release_after);
     __syncthreads();
     int64_t hits = 0;

@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256) records_kernel(EbbFlightState s, Records 
 // pass through it)
 __global__ void __launch_bounds__(256, EBB_TICK_MIN_BLOCKS) tick_kernel(EbbFlightState s, Records r) {
     __shared__ float ndt_tab[TORQUE_STEPS];
-    __shared__ float ktab[(256 / 32) * KTAB_FLOATS];
+    __shared__ float found[(256 / 32) * ORIENT_FLOATS];
     fill_ndt(ndt_tab, s.dt);
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256, EBB_TICK_MIN_BLOCKS) tick_kernel(EbbFligh
         }
         tick_begin(s, i, tgt, r.act[i] != 0, d, &release_after);
     }
-    orient_warp(d, cfg_of(s), ndt_tab, ktab + (threadIdx.x >> 5) * KTAB_FLOATS);
+    orient_warp(d, cfg_of(s), ndt_tab, found + (threadIdx.x >> 5) * ORIENT_FLOATS);
     if (mine) tick_end(s, i, d, release_after);
 }
 
@@ -262,7 +262,7 @@ __host__ __device__ inline size_t tiled_records_bytes(int cap) {
 // rows as the block has threads, so each thread ticks at most one ship.
 template <bool ONE_ROUND>
 __device__ __forceinline__ void tiled_tile(const EbbFlightState& s, int64_t r0, int64_t r1, SlotRec* rec,
-                                           const float* ndt_tab, float* ktab, int32_t* status) {
+                                           const float* ndt_tab, float* found, int32_t* status) {
     const int m = (int)(r1 - r0);
     for (int j = threadIdx.x; j < m; j += blockDim.x) {               // the records pass, into shared memory
         const int64_t i = r0 + j;
@@ -309,7 +309,7 @@ __device__ __forceinline__ void tiled_tile(const EbbFlightState& s, int64_t r0, 
             }
             tick_begin(s, i, tgt, rec[j].act != 0, d, &release_after);
         }
-        orient_warp(d, cfg_of(s), ndt_tab, ktab);
+        orient_warp(d, cfg_of(s), ndt_tab, found);
         if (mine) tick_end(s, i, d, release_after);
         if (ONE_ROUND) break;
     }
@@ -324,21 +324,21 @@ __global__ void __launch_bounds__(256, EBB_TILED_MIN_BLOCKS) tiled_kernel(EbbFli
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float ndt_tab[TORQUE_STEPS];
     SlotRec* rec = (SlotRec*)smem_raw;
-    float* ktab = (float*)(smem_raw + tiled_records_bytes(cap)) + (threadIdx.x >> 5) * KTAB_FLOATS;
+    float* found = (float*)(smem_raw + tiled_records_bytes(cap)) + (threadIdx.x >> 5) * ORIENT_FLOATS;
     fill_ndt(ndt_tab, s.dt);
     if (SINGLE) {
         if (blockIdx.x < tiles)
-            tiled_tile<true>(s, tile_rows[blockIdx.x], tile_rows[blockIdx.x + 1], rec, ndt_tab, ktab, status);
+            tiled_tile<true>(s, tile_rows[blockIdx.x], tile_rows[blockIdx.x + 1], rec, ndt_tab, found, status);
         return;
     }
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         __syncthreads();                                              // the table, and the previous tile's records
-        tiled_tile<false>(s, tile_rows[tile], tile_rows[tile + 1], rec, ndt_tab, ktab, status);
+        tiled_tile<false>(s, tile_rows[tile], tile_rows[tile + 1], rec, ndt_tab, found, status);
     }
 }
 
 __host__ __device__ inline size_t tiled_smem_bytes(int cap, int block) {
-    return tiled_records_bytes(cap) + (size_t)(block / 32) * KTAB_FLOATS * sizeof(float);
+    return tiled_records_bytes(cap) + (size_t)(block / 32) * ORIENT_FLOATS * sizeof(float);
 }
 
 // ================================================================================================ listed worlds
@@ -361,7 +361,7 @@ __host__ __device__ inline size_t listed_tables_bytes(int cap) {
     return align16((size_t)cap * sizeof(ListRec)) + align16((size_t)cap * 8) + align16((size_t)(cap + 1) * 4);
 }
 __host__ __device__ inline size_t listed_smem_bytes(int cap, int block) {
-    return listed_tables_bytes(cap) + (size_t)(block / 32) * KTAB_FLOATS * sizeof(float);
+    return listed_tables_bytes(cap) + (size_t)(block / 32) * ORIENT_FLOATS * sizeof(float);
 }
 
 // One tile of a list of worlds: world w is rows [worlds[2w], worlds[2w + 1]), the tile the worlds [w0, w0 + nw),
@@ -372,7 +372,7 @@ template <bool ONE_ROUND>
 __device__ __forceinline__ void listed_tile(const EbbFlightState& s, const int64_t* __restrict__ worlds, int64_t w0,
                                             int64_t nw64, int cap, const uint8_t* __restrict__ active,
                                             int32_t* status, ListRec* rec, int64_t* wrow, int32_t* wslot,
-                                            int* tile_rows, const float* ndt_tab, float* ktab) {
+                                            int* tile_rows, const float* ndt_tab, float* found) {
     const int lane = threadIdx.x & 31;
     if (nw64 <= 0 || nw64 > cap) {                                    // block-uniform
         if (nw64 != 0 && threadIdx.x == 0) atomicOr(status, 2);
@@ -476,7 +476,7 @@ __device__ __forceinline__ void listed_tile(const EbbFlightState& s, const int64
             }
             tick_begin(s, i, tgt, rec[j].act != 0, d, &release_after);
         }
-        orient_warp(d, cfg_of(s), ndt_tab, ktab);
+        orient_warp(d, cfg_of(s), ndt_tab, found);
         if (mine) tick_end(s, i, d, release_after);
         if (ONE_ROUND) break;
     }
@@ -497,13 +497,13 @@ __global__ void __launch_bounds__(256, EBB_TILED_MIN_BLOCKS)
     ListRec* rec = (ListRec*)smem_raw;
     int64_t* wrow = (int64_t*)(smem_raw + align16((size_t)cap * sizeof(ListRec)));
     int32_t* wslot = (int32_t*)(smem_raw + align16((size_t)cap * sizeof(ListRec)) + align16((size_t)cap * 8));
-    float* ktab = (float*)(smem_raw + listed_tables_bytes(cap)) + (threadIdx.x >> 5) * KTAB_FLOATS;
+    float* found = (float*)(smem_raw + listed_tables_bytes(cap)) + (threadIdx.x >> 5) * ORIENT_FLOATS;
     fill_ndt(ndt_tab, s.dt);
     if (SINGLE) {
         if (blockIdx.x < tiles) {
             const int64_t w0 = tile_worlds[blockIdx.x];
             listed_tile<true>(s, worlds, w0, tile_worlds[blockIdx.x + 1] - w0, cap, active, status, rec, wrow, wslot,
-                              &tile_rows, ndt_tab, ktab);
+                              &tile_rows, ndt_tab, found);
         }
         return;
     }
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(256, EBB_TILED_MIN_BLOCKS)
         __syncthreads();                                              // the previous tile's tables are done with
         const int64_t w0 = tile_worlds[tile];
         listed_tile<false>(s, worlds, w0, tile_worlds[tile + 1] - w0, cap, active, status, rec, wrow, wslot,
-                           &tile_rows, ndt_tab, ktab);
+                           &tile_rows, ndt_tab, found);
     }
 }
 

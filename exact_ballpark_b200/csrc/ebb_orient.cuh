@@ -3,14 +3,16 @@
 // GotoTorqueBreaks full.py:2155, GotoRollBreaks full.py:2224, ApplyTorque full.py:2292), warp-cooperative.
 //
 // Each torque search tries n1 = 1, 2, ... 99 accelerating ticks and keeps the first whose torque is within the
-// maximum, in up to five rounds (each round re-derives the braking ticks n2). One thread a ship runs those loops in
-// lockstep: a warp pays, round by round, its slowest ship's n1 while the others idle (about 15 % of the lanes busy on
-// the flight benchmark's worlds). Here the warp searches one ship at a time with all 32 lanes, lane j evaluating
-// candidate n1 = b + j + 1 of the block b = 0, 32, 64, 96, and a ballot takes the first candidate that passes: the
-// serial loop's n1, its alpha1 and kappa1 bit for bit, since every candidate is the same computation on the same
-// inputs (kappa1 = tf^n1 by the serial loop's own float products: kept in a per-lane table for n1 <= 32, each lane
-// carrying the chain further from the block's first kappa beyond). The set-up, the braking rounds (logf, pow) and
-// ApplyTorque stay one lane a ship, the warp's ships taking their rounds together.
+// maximum, in up to five rounds (each round re-derives the braking ticks n2): seven searches a ship and tick on the
+// flight benchmark's worlds, their n1 a median of 10 and a mean of 16. What bounds it is the issue of instructions, so the
+// searches avoid most candidates, and every lane searches for its own ship (warp_search): it guesses n1 by bisection on
+// the laws without their roundings, computes that candidate as the serial loop does (its kappa1 = tf^n1 by the serial
+// loop's own float products, every eighth of them kept), and shows that every candidate before it fails by one comparison
+// with bounds on what the serial loop's rounded operations can give (none_before). Where that does not settle a ship (one
+// in thirty), eight lanes walk its candidates, four ships at a time, each told by bounds without a division, only those
+// too near the maximum to be told computed (warp_walk). So the n1, alpha1 and kappa1 are the serial loop's, bit for bit.
+// A tick of 65,536 worlds of 4 ships: 369 us; with 32 lanes on one ship and block of 32 candidates, all computed, 584; by
+// the walk alone 636. The set-up, the braking rounds (logf, pow) and ApplyTorque are one lane a ship too.
 #pragma once
 
 #include "ebb_flight.cuh"
@@ -19,8 +21,10 @@ namespace ebb {
 namespace flight {
 
 constexpr unsigned FULL_WARP = 0xffffffffu;
-constexpr int KTAB_STRIDE = 33;             // a lane's row kappa_1 .. kappa_32 (padded: the fill is conflict-free)
-constexpr int KTAB_FLOATS = 32 * KTAB_STRIDE;
+constexpr int GROUP = 8;                    // lanes that search one ship
+constexpr int KAPPAS = 12;                  // a ship's kept kappas: kappa_8, kappa_16, ... kappa_96
+constexpr int FOUND_FLOATS = 64;            // a warp's shared memory: each ship's found n1 and kappa1,
+constexpr int ORIENT_FLOATS = FOUND_FLOATS + 32 * KAPPAS;      // and its kept kappas ([KAPPAS][32])
 
 // One lane's ship for the warp's orientation step
 struct DoLane {
@@ -41,81 +45,261 @@ __device__ __forceinline__ float wbc(float v, int src) { return __shfl_sync(FULL
 __device__ __forceinline__ int wbc(int v, int src) { return __shfl_sync(FULL_WARP, v, src); }
 __device__ __forceinline__ F3 wbc(F3 v, int src) { return F3{wbc(v.x, src), wbc(v.y, src), wbc(v.z, src)}; }
 
-// kappa1 for candidate b + lane + 1: the table for the first block, else the chain from the block's first kappa
-__device__ __forceinline__ float candidate_kappa(const float* krow, int b, int lane, float kbase, float tf) {
-    if (b == 0) return krow[lane];
-    float k = kbase;
-    for (int j = 0; j <= lane; ++j) k = fmul(k, tf);
+// Bounds on a candidate without its divisions. Write A = n2dt kappa2 / (1 - kappa2) (tau without braking ticks) and
+// u = 1 - kappa1: search_terms' num is tau - A kappa1 and its den tau (n1dt - A u) but for rounding. With each float
+// operation's relative error at most 2^-24, num as the serial loop rounds it and as computed here (one fused operation,
+// A's two) differ by less than 16 2^-24 (tau + |A| kappa1), the product by omega0 and the difference included; den by less
+// than tau 8 2^-24 (n1dt + |A| u) beside its own last rounding; and the quotient, its square and its length add less than
+// 2^-20 relatively, well inside the factors 0.998 and 1.002. Squared, (x + e)^2 <= 1.002 x^2 + 501 e^2 and
+// (x - e)^2 >= 0.998 x^2 - 500 e^2. All of it in ranges where what underflows is far below the bounds and nothing overflows
+// that the serial loop keeps (`plain` says where the bounds are not used: every candidate is then computed); a NaN decides
+// nothing.
+constexpr float NUM_ERROR = 1.0e-6f, DEN_ERROR = 5.0e-7f;      // above 16 2^-24 and 8 2^-24
+struct Bounds {
+    float A, tau, absA;
+};
+__device__ __forceinline__ bool in_range(float x, float lo, float hi) { return x >= lo && x <= hi; }
+
+// the candidate's num and den as computed here, and what the serial loop's may differ by
+__device__ __forceinline__ void candidate_terms(const Bounds& q, float k1, float n1dt, float* num, float* den, float* en,
+                                                float* ed) {
+    const float u = 1.0f - k1;
+    *num = __fmaf_rn(-q.A, k1, q.tau);
+    *den = q.tau * __fmaf_rn(-q.A, u, n1dt);
+    *en = NUM_ERROR * __fmaf_rn(q.absA, k1, q.tau);
+    *ed = DEN_ERROR * q.tau * __fmaf_rn(q.absA, u, n1dt);
+}
+// -1 the heading candidate fails, 1 it passes, 0 not told: |target - omega0 num|^2 against limit2 den^2
+__device__ __forceinline__ int tell_heading(const Bounds& q, F3 target, F3 omega0, float omega2, float limit2, float k1,
+                                            float n1dt) {
+    float num, den, en, ed;
+    candidate_terms(q, k1, n1dt, &num, &den, &en, &ed);
+    const float x = __fmaf_rn(-omega0.x, num, target.x), y = __fmaf_rn(-omega0.y, num, target.y),
+                z = __fmaf_rn(-omega0.z, num, target.z);
+    const float v2 = __fmaf_rn(x, x, __fmaf_rn(y, y, z * z)), d2 = den * den;
+    const float e2 = 520.0f * omega2 * en * en, f2 = 520.0f * ed * ed;
+    const float low = __fmaf_rn(0.998f, v2, -e2), room = limit2 * __fmaf_rn(0.998f, d2, -f2);
+    if (low > limit2 * __fmaf_rn(1.002f, d2, f2) && low > 1e-30f) return -1;
+    if (__fmaf_rn(1.002f, v2, e2) < room && room > 1e-30f) return 1;
+    return 0;
+}
+// the same of a roll candidate: |desired - omega num| against max |den|
+__device__ __forceinline__ int tell_roll(const Bounds& q, float desired, float omega, float max_alpha, float k1, float n1dt) {
+    float num, den, en, ed;
+    candidate_terms(q, k1, n1dt, &num, &den, &en, &ed);
+    const float v = fabs_(__fmaf_rn(-omega, num, desired)), d = fabs_(den), e = fabs_(omega) * en;
+    const float low = __fmaf_rn(0.998f, v, -e), room = max_alpha * __fmaf_rn(0.998f, d, -ed);
+    if (low > max_alpha * __fmaf_rn(1.002f, d, ed) && low > 1e-20f) return -1;
+    if (__fmaf_rn(1.002f, v, e) < room && room > 1e-20f) return 1;
+    return 0;
+}
+
+// One ship's search as its lane sets it up
+struct Quest {
+    Search q;
+    float tf, max_alpha, limit2;
+    bool squared;
+    F3 target, omega0;                      // the heading's; a roll's desired angle and turning rate in x
+};
+// alpha1 and whether it is within the maximum, as the serial loop computes them (full.py:2189-2201, 2264-2276; the roll's
+// by a true division)
+template <bool ROLL>
+__device__ __forceinline__ bool candidate(const Quest& s, float k1, float n1dt, F3* a1) {
+    float num, den;
+    search_terms(s.q, k1, n1dt, &num, &den);
+    if (ROLL) {
+        a1->x = fdiv(fsub(s.target.x, fmul(s.omega0.x, num)), den);
+        return fabs_(a1->x) < s.max_alpha;
+    }
+    *a1 = f3_div(f3_sub(s.target, f3_mul(s.omega0, num)), den);
+    return s.squared ? f3_dot(*a1, *a1) < s.limit2 : f3_len(*a1) < s.max_alpha;
+}
+
+// The searches of the lanes in `want` candidate by candidate, four ships at a time, eight lanes a ship: each lane's n1 and
+// kappa1 (n1 = 100 with the 99th candidate's kappa1 when none passes), and its alpha1, left in that lane
+template <bool ROLL>
+__device__ __forceinline__ void warp_walk(unsigned want, const Quest& mine, const Bounds& mine_bd, float o2, bool plain,
+                                          const float* ndt_tab, float* found, int* n1_out, F3* a1_out, float* k1_out) {
+    const int lane = threadIdx.x & 31, sub = lane & (GROUP - 1), first = lane & ~(GROUP - 1);
+    const unsigned group = ((1u << GROUP) - 1u) << first;
+    const bool searching = (want >> lane) & 1;
+    while (want) {
+        unsigned m = want;                                   // the next four ships, one a group
+        int src = -1;
+#pragma unroll
+        for (int g = 0; g < 32 / GROUP; ++g) {
+            const int k = __ffs(m) - 1;
+            if (g == (lane / GROUP)) src = k;
+            m &= m - 1;
+        }
+        want = m;
+        const int from = src < 0 ? lane : src;
+        Bounds bd;
+        bd.A = wbc(mine_bd.A, from);
+        bd.tau = wbc(mine.q.tau, from);
+        bd.absA = fabs_(bd.A);
+        const float tf = wbc(mine.tf, from), max_alpha = wbc(mine.max_alpha, from);
+        float limit2 = 0.0f, omega2 = 0.0f;
+        F3 target, omega0;
+        if (ROLL) {
+            target.x = wbc(mine.target.x, from);
+            omega0.x = wbc(mine.omega0.x, from);
+        } else {
+            target = wbc(mine.target, from);
+            omega0 = wbc(mine.omega0, from);
+            limit2 = wbc(mine.limit2, from);
+            omega2 = wbc(o2, from);
+        }
+        const bool untold = wbc((int)plain, from) != 0;
+        float k1 = tf;                                       // kappa_{sub + 1}
+#pragma unroll
+        for (int i = 1; i < GROUP; ++i)
+            if (i <= sub) k1 = fmul(k1, tf);
+        bool open = src >= 0;
+        for (int b = 0;; b += GROUP) {
+            const int n = b + sub + 1;
+            const float n1dt = ndt_tab[n < TORQUE_STEPS ? n : TORQUE_STEPS - 1];
+            int told = 0;
+            if (!untold)
+                told = ROLL ? tell_roll(bd, target.x, omega0.x, max_alpha, k1, n1dt)
+                            : tell_heading(bd, target, omega0, omega2, limit2, k1, n1dt);
+            if (n >= TORQUE_STEPS) told = -1;
+            unsigned maybe = __ballot_sync(FULL_WARP, open && told >= 0) & group;
+            const bool doubt = maybe != 0 && lane == __ffs(maybe) - 1 && told == 0;
+            if (__any_sync(FULL_WARP, doubt)) {              // a group's first is not told: its candidates are computed
+                Quest s;
+                s.q.tau = bd.tau;
+                s.q.n2 = wbc(mine.q.n2, from);
+                s.q.kappa2 = wbc(mine.q.kappa2, from);
+                s.q.n2dt = wbc(mine.q.n2dt, from);
+                s.q.one_k2 = wbc(mine.q.one_k2, from);
+                s.tf = tf;
+                s.max_alpha = max_alpha;
+                s.limit2 = limit2;
+                s.squared = wbc((int)mine.squared, from) != 0;
+                s.target = target;
+                s.omega0 = omega0;
+                F3 a1;
+                if (told == 0) told = candidate<ROLL>(s, k1, n1dt, &a1) ? 1 : -1;
+                maybe = __ballot_sync(FULL_WARP, open && told > 0) & group;
+            }
+            const bool last = b + GROUP >= TORQUE_STEPS - 1;
+            if (open && (maybe || last)) {
+                // the first that passes (every one before it fails), or the 99th
+                const int w = maybe ? __ffs(maybe) - 1 : first + (TORQUE_STEPS - 2 - b);
+                if (lane == w) {
+                    found[2 * src] = __int_as_float(maybe ? n : TORQUE_STEPS);
+                    found[2 * src + 1] = k1;
+                }
+                open = false;
+            }
+            if (!__any_sync(FULL_WARP, open)) break;
+#pragma unroll
+            for (int i = 0; i < GROUP; ++i) k1 = fmul(k1, tf);
+        }
+    }
+    __syncwarp();
+    if (searching) {
+        const int n1 = __float_as_int(found[2 * lane]);
+        const float k1 = found[2 * lane + 1];
+        candidate<ROLL>(mine, k1, ndt_tab[n1 < TORQUE_STEPS ? n1 : TORQUE_STEPS - 1], a1_out);
+        *n1_out = n1;
+        *k1_out = k1;
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ float exp2_near(float x) {
+    float y;
+    asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// kappa_n exactly, n < 100: the kept one below it and the products from there
+__device__ __forceinline__ float kappa_at(const float* kept, int n, float tf) {
+    const int b = n / GROUP, r = n % GROUP;
+    float k = b ? kept[(b - 1) * 32] : 1.0f;
+#pragma unroll
+    for (int i = 1; i < GROUP; ++i)
+        if (i <= r) k = fmul(k, tf);
     return k;
 }
-
-// The heading search's round for one ship (the loop of full.py:2189-2201), all lanes: the first n1 in 1 .. 99 whose
-// alpha1 = (target - omega0 num) / den is within max_alpha (n1 = 100 with the 99th candidate when none is), and its
-// alpha1 and kappa1, returned to every lane
-__device__ __forceinline__ void warp_search_v(const float* krow, const float* ndt_tab, F3 target, F3 omega0,
-                                           const Search& q, float tf, float max_alpha, float limit2, bool squared,
-                                           int lane, int* n1_out, F3* a1_out, float* k1_out) {
-    float kbase = 1.0f;
-    for (int b = 0;; b += 32) {
-        const int cand = b + lane + 1;
-        const float k1 = candidate_kappa(krow, b, lane, kbase, tf);
-        float num, den;
-        search_terms(q, k1, ndt_tab[cand < TORQUE_STEPS ? cand : TORQUE_STEPS - 1], &num, &den);
-        const F3 a1 = f3_div(f3_sub(target, f3_mul(omega0, num)), den);
-        const bool pass = squared ? (f3_dot(a1, a1) < limit2) : (f3_len(a1) < max_alpha);
-        const unsigned hit = __ballot_sync(FULL_WARP, cand < TORQUE_STEPS && pass);
-        if (hit) {
-            const int first = __ffs(hit) - 1;
-            *n1_out = b + first + 1;
-            *a1_out = wbc(a1, first);
-            *k1_out = wbc(k1, first);
-            return;
-        }
-        if (b + 32 >= TORQUE_STEPS - 1) {                            // none passes: n1 = 100, the 99th's values
-            const int last = TORQUE_STEPS - 2 - b;
-            *n1_out = TORQUE_STEPS;
-            *a1_out = wbc(a1, last);
-            *k1_out = wbc(k1, last);
-            return;
-        }
-        kbase = wbc(k1, 31);
+// Whether every candidate 1 .. n fails, told at once: num rises with n (kappa1 falls) from `first`, so the least
+// |target - omega0 num| is at num's nearest to the line's foot (the same roll: where the coast ends on the target); den rises with n but for what the kappas' own rounding takes back, at most
+// |A| (1 - tf + 2^-23) - dt a candidate.
+template <bool ROLL>
+__device__ __forceinline__ bool none_before(const Bounds& q, const Quest& s, float o2, float first, float foot, float kn,
+                                            int n, float ndt_n, float dt) {
+    const float num = fminf(fmaxf(foot, first), __fmaf_rn(-q.A, kn, q.tau));
+    const float en = NUM_ERROR * (q.tau + q.absA);
+    const float back = fmaxf(0.0f, __fmaf_rn(q.absA, (1.0f - s.tf) + 1.3e-7f, -dt)) * (float)n * 1.01f;
+    const float u = 1.0f - kn;
+    const float d = q.tau * (fabs_(__fmaf_rn(-q.A, u, ndt_n)) + back), ed = DEN_ERROR * q.tau * __fmaf_rn(q.absA, u, ndt_n);
+    if (ROLL) {
+        const float v = fabs_(__fmaf_rn(-s.omega0.x, num, s.target.x)), e = fabs_(s.omega0.x) * en;
+        const float low = __fmaf_rn(0.998f, v, -e);
+        return low > s.max_alpha * __fmaf_rn(1.002f, d, ed) && low > 1e-20f;
     }
+    const float x = __fmaf_rn(-s.omega0.x, num, s.target.x), y = __fmaf_rn(-s.omega0.y, num, s.target.y),
+                z = __fmaf_rn(-s.omega0.z, num, s.target.z);
+    const float v2 = __fmaf_rn(x, x, __fmaf_rn(y, y, z * z));
+    const float low = __fmaf_rn(0.998f, v2, -520.0f * o2 * en * en);
+    return low > s.limit2 * __fmaf_rn(1.002f, d * d, 520.0f * ed * ed) && low > 1e-30f;
 }
 
-// The roll search's round for one ship (full.py:2264-2276): a true division, |alpha1| against max_alpha
-__device__ __forceinline__ void warp_search_f(const float* krow, const float* ndt_tab, float desired, float omega_roll,
-                                           const Search& q, float tf, float max_alpha, int lane, int* n1_out,
-                                           float* a1_out, float* k1_out) {
-    float kbase = 1.0f;
-    for (int b = 0;; b += 32) {
-        const int cand = b + lane + 1;
-        const float k1 = candidate_kappa(krow, b, lane, kbase, tf);
-        float num, den;
-        search_terms(q, k1, ndt_tab[cand < TORQUE_STEPS ? cand : TORQUE_STEPS - 1], &num, &den);
-        const float a1 = fdiv(fsub(desired, fmul(omega_roll, num)), den);
-        const unsigned hit = __ballot_sync(FULL_WARP, cand < TORQUE_STEPS && fabs_(a1) < max_alpha);
-        if (hit) {
-            const int first = __ffs(hit) - 1;
-            *n1_out = b + first + 1;
-            *a1_out = wbc(a1, first);
-            *k1_out = wbc(k1, first);
-            return;
-        }
-        if (b + 32 >= TORQUE_STEPS - 1) {
-            const int last = TORQUE_STEPS - 2 - b;
-            *n1_out = TORQUE_STEPS;
-            *a1_out = wbc(a1, last);
-            *k1_out = wbc(k1, last);
-            return;
-        }
-        kbase = wbc(k1, 31);
-    }
-}
-
-// The warp's orientation step: every lane calls it together (lanes whose ship is off pass through). `ktab` is the
-// warp's KTAB_FLOATS floats of shared memory; `ndt_tab` the block's table float(n dt).
-__device__ __forceinline__ void orient_warp(DoLane& d, const Cfg& c, const float* ndt_tab, float* ktab) {
+// The round's searches of the lanes in `want`: each searching lane's n1, kappa1 and alpha1. A lane guesses its own ship's
+// n1 by bisection on the laws without their roundings, num's best so far in place of num, so that a passing candidate is
+// followed by passing ones alone; computes that candidate as the serial loop does, and tells by bounds whether every one before it fails; the ships for
+// which the two don't settle it are walked.
+template <bool ROLL>
+__device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, const float* ndt_tab, float* found, float dt,
+                                            int* n1_out, F3* a1_out, float* k1_out) {
     const int lane = threadIdx.x & 31;
+    const float* kept = found + FOUND_FLOATS + lane;
+    bool settled = true;
+    Bounds bd;
+    float o2 = 0.0f;
+    bool plain = false;
+    if ((want >> lane) & 1) {
+        bd.tau = bd.A = mine.q.tau;
+        if (mine.q.n2 != 0) bd.A = fdiv(fmul(mine.q.n2dt, mine.q.kappa2), mine.q.one_k2);
+        bd.absA = fabs_(bd.A);
+        o2 = f3_dot(mine.omega0, mine.omega0);
+        const float t2 = f3_dot(mine.target, mine.target), to = f3_dot(mine.target, mine.omega0);
+        plain = !(in_range(mine.q.tau, 1e-8f, 1e8f) && bd.absA <= 1e8f && in_range(mine.tf, 0.0f, 1.0f) &&
+                  (ROLL ? in_range(mine.max_alpha, 1e-8f, 1e8f) : mine.squared && in_range(mine.limit2, 1e-16f, 1e16f)) &&
+                  t2 < 1e8f && o2 < 1e8f && in_range(dt, 1e-4f, 1e4f));
+        settled = false;
+        if (!plain) {
+            const float l2 = __log2f(mine.tf), m2 = ROLL ? mine.max_alpha * mine.max_alpha : mine.limit2;
+            const float first = __fmaf_rn(-bd.A, mine.tf, bd.tau), foot = __fdividef(to, o2);
+            int below = 0, n = TORQUE_STEPS;
+#pragma unroll 1
+            while (n - below > 1) {
+                const int mid = (below + n) >> 1;
+                const float nf = (float)mid, k = exp2_near(nf * l2), u = 1.0f - k;
+                const float num = __fmaf_rn(-bd.A, k, bd.tau), den = bd.tau * __fmaf_rn(-bd.A, u, nf * dt);
+                const float near = fminf(fmaxf(foot, first), num);   // (num's best up to there: so a pass stays one)
+                const bool pass = __fmaf_rn(__fmaf_rn(o2, near, -2.0f * to), near, t2) < m2 * den * den;
+                below = pass ? below : mid;
+                n = pass ? mid : n;
+            }
+            const float kb = kappa_at(kept, n - 1, mine.tf);
+            const bool none = n == TORQUE_STEPS;             // (then the 99th's values)
+            const float k1 = none ? kb : fmul(kb, mine.tf);
+            const bool pass = candidate<ROLL>(mine, k1, ndt_tab[none ? n - 1 : n], a1_out);
+            settled = (none ? !pass : pass) &&
+                      (n == 1 || none_before<ROLL>(bd, mine, o2, first, foot, kb, n - 1, ndt_tab[n - 1], dt));
+            *n1_out = n;
+            *k1_out = k1;
+        }
+    }
+    const unsigned open = __ballot_sync(FULL_WARP, !settled);
+    if (open) warp_walk<ROLL>(open, mine, bd, o2, plain, ndt_tab, found, n1_out, a1_out, k1_out);
+}
+
+// The warp's orientation step: every lane calls it together (lanes whose ship is off pass through). `found` is the
+// warp's ORIENT_FLOATS floats of shared memory; `ndt_tab` the block's table float(n dt).
+__device__ __forceinline__ void orient_warp(DoLane& d, const Cfg& c, const float* ndt_tab, float* found) {
     const F3 zero = F3{0.0f, 0.0f, 0.0f};
     d.torque = zero;
     d.roll = 0.0f;
@@ -141,10 +325,12 @@ __device__ __forceinline__ void orient_warp(DoLane& d, const Cfg& c, const float
         t.fdt = c.fdt;
         t.ndt_tab = ndt_tab;
         a32 = f3_of(d.a);
-        float k = 1.0f;                                               // kappa_1 .. kappa_32, as the loops form them
-        for (int j = 0; j < 32; ++j) {
-            k = fmul(k, t.tf);
-            ktab[lane * KTAB_STRIDE + j] = k;
+        float k = 1.0f;                                               // the kept kappas, as the loops form them
+        float* kept = found + FOUND_FLOATS + (threadIdx.x & 31);
+        for (int b = 0; b < KAPPAS; ++b) {
+#pragma unroll
+            for (int i = 0; i < GROUP; ++i) k = fmul(k, t.tf);
+            kept[b * 32] = k;
         }
     }
     __syncwarp();
@@ -198,28 +384,10 @@ __device__ __forceinline__ void orient_warp(DoLane& d, const Cfg& c, const float
                 }
             }
         }
-        unsigned want = __ballot_sync(FULL_WARP, h_active);
+        const unsigned want = __ballot_sync(FULL_WARP, h_active);
         if (!want) break;
-        while (want) {
-            const int k = __ffs(want) - 1;
-            want &= want - 1;
-            Search qk;
-            qk.tau = wbc(q.tau, k);
-            qk.n2 = wbc(q.n2, k);
-            qk.kappa2 = wbc(q.kappa2, k);
-            qk.n2dt = wbc(q.n2dt, k);
-            qk.one_k2 = wbc(q.one_k2, k);
-            int n1;
-            F3 a1;
-            float k1;
-            warp_search_v(ktab + k * KTAB_STRIDE, ndt_tab, wbc(h_target, k), wbc(h_omega0, k), qk, wbc(t.tf, k),
-                          wbc(h_max, k), wbc(h_limit2, k), wbc((int)h_sq, k) != 0, lane, &n1, &a1, &k1);
-            if (lane == k) {
-                h_n1 = n1;
-                h_alpha1 = a1;
-                h_kappa1 = k1;
-            }
-        }
+        const Quest mine{q, t.tf, h_max, h_limit2, h_sq, h_target, h_omega0};
+        warp_search<false>(want, mine, ndt_tab, found, c.fdt, &h_n1, &h_alpha1, &h_kappa1);
         if (h_active) {
             const F3 omega1 = f3_add(f3_mul(h_alpha1, fmul(t.tau_s, fsub(1.0f, h_kappa1))), f3_mul(h_omega0, h_kappa1));
             const int n2_old = h_n2;
@@ -285,27 +453,12 @@ __device__ __forceinline__ void orient_warp(DoLane& d, const Cfg& c, const float
                 }
             }
         }
-        unsigned want = __ballot_sync(FULL_WARP, r_active);
+        const unsigned want = __ballot_sync(FULL_WARP, r_active);
         if (!want) break;
-        while (want) {
-            const int k = __ffs(want) - 1;
-            want &= want - 1;
-            Search qk;
-            qk.tau = wbc(q.tau, k);
-            qk.n2 = wbc(q.n2, k);
-            qk.kappa2 = wbc(q.kappa2, k);
-            qk.n2dt = wbc(q.n2dt, k);
-            qk.one_k2 = wbc(q.one_k2, k);
-            int n1;
-            float a1, k1;
-            warp_search_f(ktab + k * KTAB_STRIDE, ndt_tab, wbc(r_desired, k), wbc(r_omega, k), qk, wbc(t.tf, k),
-                          wbc(r_max, k), lane, &n1, &a1, &k1);
-            if (lane == k) {
-                r_n1 = n1;
-                r_alpha1 = a1;
-                r_kappa1 = k1;
-            }
-        }
+        const Quest mine{q, t.tf, r_max, 0.0f, false, F3{r_desired, 0.0f, 0.0f}, F3{r_omega, 0.0f, 0.0f}};
+        F3 a1 = zero;
+        warp_search<true>(want, mine, ndt_tab, found, c.fdt, &r_n1, &a1, &r_kappa1);
+        if (r_active) r_alpha1 = a1.x;
         if (r_active) {
             const float omega1 = fadd(fmul(fmul(r_alpha1, t.tau_s), fsub(1.0f, r_kappa1)), fmul(r_omega, r_kappa1));
             const int n2_old = r_n2;
