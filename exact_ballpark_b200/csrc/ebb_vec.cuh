@@ -93,13 +93,16 @@ __device__ __forceinline__ M3 m_of_q(F4 q) {
     return m;
 }
 // TransformCoord: the row vector (v, 1) times the matrix, divided by its w (the 0 0 0 1 column keeps every zero's
-// sign through the sums)
+// sign through the sums). The w is exactly 1 unless v holds an infinity or a NaN, and a division by 1 leaves its operand:
+// so a finite v takes none (three IEEE divisions a call, seven calls a ship and tick with dynamical orientation).
 __device__ __forceinline__ F3 m_apply(F3 v, const M3& m) {
     const float norm = fadd(fadd(fadd(fmul(0.0f, v.x), fmul(0.0f, v.y)), fmul(0.0f, v.z)), 1.0f);
     if (!(norm != 0.0f)) return F3{0.0f, 0.0f, 0.0f};
-    return F3{fdiv(fadd(fadd(fadd(fmul(v.x, m.r0.x), fmul(v.y, m.r1.x)), fmul(v.z, m.r2.x)), 0.0f), norm),
-              fdiv(fadd(fadd(fadd(fmul(v.x, m.r0.y), fmul(v.y, m.r1.y)), fmul(v.z, m.r2.y)), 0.0f), norm),
-              fdiv(fadd(fadd(fadd(fmul(v.x, m.r0.z), fmul(v.y, m.r1.z)), fmul(v.z, m.r2.z)), 0.0f), norm)};
+    F3 r = F3{fadd(fadd(fadd(fmul(v.x, m.r0.x), fmul(v.y, m.r1.x)), fmul(v.z, m.r2.x)), 0.0f),
+              fadd(fadd(fadd(fmul(v.x, m.r0.y), fmul(v.y, m.r1.y)), fmul(v.z, m.r2.y)), 0.0f),
+              fadd(fadd(fadd(fmul(v.x, m.r0.z), fmul(v.y, m.r1.z)), fmul(v.z, m.r2.z)), 0.0f)};
+    if (norm != 1.0f) r = F3{fdiv(r.x, norm), fdiv(r.y, norm), fdiv(r.z, norm)};
+    return r;
 }
 
 }  // namespace ebb
