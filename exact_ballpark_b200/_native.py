@@ -136,6 +136,7 @@ def lib() -> ctypes.CDLL:
     L.ebb_collide_tick.argtypes = [p, p, p, p]
     L.ebb_collide_load.argtypes = [p, p, p]
     L.ebb_combat_tick.argtypes = [ctypes.POINTER(CombatState), p, i64, p, p, i32]
+    L.ebb_combat_watch.argtypes = [ctypes.POINTER(CombatState), p, i64, i64, p]
     L.ebb_composed_tick.argtypes = [ctypes.POINTER(ComposedState), p, i64, p, p, i32]
     L.ebb_composed_file.argtypes = [ctypes.POINTER(ComposedState), p, p, p, p, p]
     L.ebb_server_tick.argtypes = [ctypes.POINTER(ServerState), ctypes.POINTER(ServerQueue), i32, i64, i64, p, i32]

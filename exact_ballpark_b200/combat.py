@@ -526,11 +526,12 @@ class VecCombatPark(VecModesPark):
 
     def watch(self) -> None:
         """A world holding two massive balls outside MISSILE mode is flagged on all its rows: this park computes only
-        a normal missile's contact with its target (index work on the device)."""
-        m = self._exists & ~self._moribund & self._massive & (self._mode != MISSILE)
+        a normal missile's contact with its target (one launch)."""
         rw = self.rows_of_world
-        two = (m[rw.clamp(min=0)] & (rw >= 0)).sum(dim=1) > 1
-        self._flags |= torch.where(two[self.world_index], FLAG_MASSIVE, 0)
+        with torch.cuda.device(self.dev):
+            rc = _native.lib().ebb_combat_watch(ctypes.byref(self.combat_state()), rw.data_ptr(), rw.shape[0], rw.shape[1],
+                                                self._stream())
+        _native.check(rc, "ebb_combat_watch")
 
     def world_flags(self) -> list:
         """Each world's flags (the OR of its rows'), in world label order."""

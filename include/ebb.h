@@ -75,6 +75,7 @@ typedef struct EbbCollideState {
  * the leader's formation (char semantics, -1 none) and slot bits, a missile's owner row (-1 none), the tick's
  * contact and dispatch counts, and the bubble and cloak the commands keep; the formation table [formations][max
  * slots][3] with each formation's length. Dynamical orientation is required (flight.dynamical = 1). */
+#define EBB_COMBAT_FLAG_MASSIVE 32
 typedef struct EbbCombatState {
     EbbFlightState flight;
     uint8_t* exists;
@@ -361,6 +362,11 @@ int ebb_collide_load(const EbbCollideState* s, int32_t* status, void* stream);
  * and commit launches), which exact_ballpark.vec_combat_cuda.tick calls (vec_combat_cuda.py:289). */
 int ebb_combat_tick(const EbbCombatState* s, const int64_t* tile_rows, int64_t tiles, int32_t* status, void* stream,
                     int block);
+
+/* The combat park's domain watch: EBB_COMBAT_FLAG_MASSIVE raised on every row of a world that holds two massive balls in
+ * the park outside MISSILE mode. `rows` [worlds][width]: each world's rows, -1 padded. Replaces VecCombatPark.watch
+ * (vec_combat.py:1043). */
+int ebb_combat_watch(const EbbCombatState* s, const int64_t* rows, int64_t worlds, int64_t width, void* stream);
 
 /* One tick of the composed park in place, in tiles of whole worlds as ebb_combat_tick: the records pass, phase 1 (the
  * live balls' collision lists cleared), the warp paths with the drop-outs (re-filed at rest), the gradient for every
