@@ -257,6 +257,14 @@ __host__ __device__ inline size_t tiled_records_bytes(int cap) {
     return ((size_t)cap * sizeof(SlotRec) + 15) & ~(size_t)15;
 }
 
+// The rows a warp of a one-round tile of m rows takes: an even share, 32 in a full tile. A plan of few rows has tiles of
+// fewer rows than threads (tiles.py: shape_for): with 32 ships a warp pays for every mode, search and walk among them
+// while most of the chip waits.
+__device__ __forceinline__ int rows_a_warp(int m) {
+    const int warps = blockDim.x >> 5, per = (m + warps - 1) / warps;
+    return per < 32 ? per : 32;
+}
+
 // One tile (a run of whole worlds, rows [r0, r1)): the records pass into shared memory, then the tile's ships' ticks,
 // each warp taking 32 ships at a time through the warp's orientation step. ONE_ROUND: the tile has at most as many
 // rows as the block has threads, so each thread ticks at most one ship.
@@ -283,9 +291,10 @@ __device__ __forceinline__ void tiled_tile(const EbbFlightState& s, int64_t r0, 
         q.act = act ? 1 : 0;
     }
     __syncthreads();
-    for (int base = threadIdx.x & ~31; base < m; base += blockDim.x) {   // warp-uniform: each warp's 32 ships
+    const int per = ONE_ROUND ? rows_a_warp(m) : 32;
+    for (int base = (int)(threadIdx.x >> 5) * per; base < m; base += blockDim.x) {   // warp-uniform: each warp's ships
         const int j = base + (threadIdx.x & 31);
-        const bool mine = j < m;
+        const bool mine = j < m && j < base + per;
         DoLane d;
         d.on = false;
         bool release_after = false;
@@ -443,9 +452,10 @@ __device__ __forceinline__ void listed_tile(const EbbFlightState& s, const int64
         q.world = lo;
     }
     __syncthreads();
-    for (int base = threadIdx.x & ~31; base < m; base += blockDim.x) {   // warp-uniform: each warp's 32 slots
+    const int per = ONE_ROUND ? rows_a_warp(m) : 32;
+    for (int base = (int)(threadIdx.x >> 5) * per; base < m; base += blockDim.x) {   // warp-uniform: each warp's slots
         const int j = base + lane;
-        bool mine = j < m;
+        bool mine = j < m && j < base + per;
         int64_t i = 0;
         int e = 0;
         if (mine) {

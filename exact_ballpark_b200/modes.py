@@ -31,7 +31,7 @@ import numpy as np
 import torch
 
 from . import _native
-from .tiles import TilePlan, plan_tiles
+from .tiles import TilePlan, plan_for
 
 F64, F32, I64, I32, BOOL = torch.float64, torch.float32, torch.int64, torch.int32, torch.bool
 
@@ -289,7 +289,7 @@ class VecModesPark:
         self._decay_rows(every)
         if self.dynamical_orientation:
             self._snap(every, fresh=True)
-        self.plan = plan_tiles(self.world)
+        self.plan = plan_for(self.world)
 
     # ---- the follower bookkeeping: Stop(Ball*) (vec_modes.py:289) ----
     def _following(self) -> torch.Tensor:

@@ -41,6 +41,7 @@ import torch
 
 from . import _native
 from .modes import _STATE_FIELD, _STORAGE, VecModesPark
+from .tiles import shape_for
 from .workloads import FlightWorlds, PackedWorlds, flight_worlds, ragged_ships
 
 STATE_BYTES_PER_ROW = sum((8 if dt in (torch.float64, torch.int64) else 4 if dt in (torch.float32, torch.int32) else 1)
@@ -331,7 +332,7 @@ class Server:
         self.tile_cap, self.block = int(tile_cap), int(block)
         self.grid = grid
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
-        self._plan = None                        # (worlds, tile_worlds, tiles) on the device
+        self._plan = None                        # (worlds, tile_worlds on the device, tiles, cap, block)
         self._dirty = True
         self.table = LiveTable()
         self.ends: dict = {}                     # step -> eids whose last tick it is
@@ -450,19 +451,24 @@ class Server:
         c = self.table.count
         main = torch.cuda.current_stream(self.dev)
         wb, tb = self.up_worlds.buffer(2 * c), self.up_tiles.buffer(c + 1)
-        worlds, tile_worlds = plan_worlds(self.table.start[:c], self.table.len[:c], self.tile_cap, wb, tb)
+        cap, block = self.tile_cap, self.block
+        if c:                                             # tiles and blocks no larger than the live rows ask for
+            small, threads = shape_for(self.live_rows, int(self.table.len[:c].max()))
+            if small <= cap and self.grid is None:
+                cap, block = small, min(block, threads)
+        worlds, tile_worlds = plan_worlds(self.table.start[:c], self.table.len[:c], cap, wb, tb)
         self._plan = (self.up_worlds.send(len(worlds), main), self.up_tiles.send(len(tile_worlds), main),
-                      len(tile_worlds) - 1)
+                      len(tile_worlds) - 1, cap, block)
         self._dirty = False
 
     def _tick(self) -> int:
-        worlds, tile_worlds, tiles = self._plan
+        worlds, tile_worlds, tiles, cap, block = self._plan
         if tiles <= 0:
             return 0
         grid = tiles if self.grid is None else min(tiles, self.grid)
         rc = _native.lib().ebb_flight_tick_worlds(
-            ctypes.byref(self.park.state()), worlds.data_ptr(), tile_worlds.data_ptr(), tiles, self.tile_cap, None,
-            self.status.data_ptr(), torch.cuda.current_stream(self.dev).cuda_stream, self.block, grid)
+            ctypes.byref(self.park.state()), worlds.data_ptr(), tile_worlds.data_ptr(), tiles, cap, None,
+            self.status.data_ptr(), torch.cuda.current_stream(self.dev).cuda_stream, block, grid)
         _native.check(rc, "ebb_flight_tick_worlds")
         return self.live_rows
 

@@ -85,12 +85,43 @@ def pack(runs: list, cap: int) -> list:
 def plan_tiles(world: torch.Tensor, cap: int = DEFAULT_CAP, block: int | None = None, grid: int | None = None):
     """The tile plan for a park's world column, or None when its worlds are not contiguous runs or a world is larger
     than MAX_CAP rows."""
-    runs = world_runs(world)
+    return _plan(world_runs(world), lambda n, max_world: (cap, block), grid)
+
+
+def plan_for(world: torch.Tensor):
+    """plan_tiles with the shape the park's size asks for (shape_for)."""
+    return _plan(world_runs(world), shape_for, None)
+
+
+# The least warps a park's rows are spread over: one a scheduler of the chip's 148 multiprocessors
+SPREAD_WARPS = 592
+
+
+def shape_for(rows: int, max_world: int) -> tuple:
+    """The (cap, block) of a one-tile-a-block plan for `rows` rows whose largest world has max_world. A warp's time grows
+    with its ships (their modes, their searches, the slowest of them), so few rows are spread over the chip, 4 to 32 a
+    warp, until each of its schedulers has a warp; more rows take full warps, in blocks of 128 threads (their ends even
+    out over the multiprocessors) until a wave of 256-thread blocks is full (their warps share the instruction cache).
+    Dynamical orientation on, us a tick, as 256-row tiles and so: 64 worlds of 4 ships 64 and 52, 600 72 and 62, 2,000 73
+    and 67, 5,000 77 and 74, 20,000 115 and 105, 65,536 344 and 344 (128-thread blocks: 367); 100 worlds of 1 to 128 ships
+    75 and 69. Without it every shape of 64 worlds takes 14."""
+    warp = 4
+    while warp < 32 and rows > warp * SPREAD_WARPS:
+        warp *= 2
+    if warp == 32:
+        block = 256 if rows >= 3 * 148 * 256 else 128
+        return max(block, max_world), (block if max_world <= block else 256)
+    cap = max(warp, max_world)
+    return cap, min(256, 32 * ((cap + warp - 1) // warp))
+
+
+def _plan(runs: list | None, shape, grid: int | None):
     if runs is None or len(runs) < 2:
         return None
     max_world = max(b - a for a, b in zip(runs[:-1], runs[1:]))
     if max_world > MAX_CAP:
         return None
+    cap, block = shape(runs[-1], max_world)
     cap = min(max(cap, max_world), MAX_CAP)
     tile_rows = pack(runs, cap)
     blk = block or DEFAULT_BLOCK
