@@ -124,14 +124,29 @@ class RowSpace:
 
 class Rows:
     """Rows of park state in the park's device layout with no park behind them (finished episodes' final states): the
-    storage tensors `_<name>`, `field()` in the reference layout, and `state()` for the native calls."""
+    storage tensors `_<name>`, `field()` in the reference layout, and `state()` for the native calls. The fields share one
+    buffer, each from a 256-byte boundary, and a field's tensor is made when it is first asked for: a retirement makes one
+    allocation where a tensor a field made 34 (half of the loop's host time when every step retires something)."""
 
     def __init__(self, n: int, like: VecModesPark):
         self.n, self.dev = int(n), like.dev
+        self._at, size = {}, 0
         for name, dt, planes in _STORAGE:
-            setattr(self, "_" + name, torch.empty((planes, n) if planes else (n,), dtype=dt, device=like.dev))
+            self._at["_" + name] = (size, dt, planes)
+            size += (max(planes, 1) * self.n * dt.itemsize + 255) // 256 * 256
+        self._buffer = torch.empty(size, dtype=torch.uint8, device=like.dev)
         self._like = like
         self._state = None
+
+    def __getattr__(self, name: str):                     # (a field's tensor, the first time)
+        at = self.__dict__.get("_at", {}).get(name)
+        if at is None:
+            raise AttributeError(name)
+        off, dt, planes = at
+        t = self._buffer[off:off + max(planes, 1) * self.n * dt.itemsize].view(dt)
+        t = t.reshape(planes, self.n) if planes else t
+        setattr(self, name, t)
+        return t
 
     def state(self) -> _native.FlightState:
         if self._state is None:
@@ -139,8 +154,9 @@ class Rows:
             lk = self._like.state()
             s.n, s.friction, s.dt, s.ffriction, s.fdt = self.n, lk.friction, lk.dt, lk.ffriction, lk.fdt
             s.new_orbit, s.dynamical = lk.new_orbit, lk.dynamical
+            base = self._buffer.data_ptr()
             for name, _, _ in _STORAGE:
-                setattr(s, _STATE_FIELD.get(name, name), getattr(self, "_" + name).data_ptr())
+                setattr(s, _STATE_FIELD.get(name, name), base + self._at["_" + name][0])
             self._state = s
         return self._state
 
@@ -191,9 +207,9 @@ class Uploads:
         """The first n entries of the buffer just written, on the device (queued on `stream`)."""
         dst = self.device[:n]
         dst.copy_(self.host[self.turn][:n], non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record(stream)
-        self.done[self.turn] = ev
+        if self.done[self.turn] is None:
+            self.done[self.turn] = torch.cuda.Event()
+        self.done[self.turn].record(stream)               # (its previous copy was waited for when the buffer was taken)
         return dst
 
     def put(self, a: np.ndarray, stream) -> torch.Tensor:
