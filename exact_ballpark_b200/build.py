@@ -22,11 +22,10 @@ SOURCES = ("ebb_flight.cu", "ebb_collide.cu", "ebb_combat.cu", "ebb_server.cu", 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-fmad=false",
               "-prec-div=true", "-prec-sqrt=true", "-ftz=false", "-Xcompiler", "-fPIC,-ffp-contract=off,-fno-fast-math",
               "-Xptxas", "-v", "-shared"]
-# per source: the space layer's program is long, branchy and latency-bound (a sequential program a world), and
-# ptxas's -O1 schedule of it runs a few per cent faster on the B200 than -O3's (measured on the partition workload);
-# the flight ticks' kernels are instruction-fetch-bound, and -O1's shorter code ran the tiled tick 7 % faster
-# (65,536 worlds x 4 ships, dynamical orientation: 0.433 against 0.462 ms)
-SOURCE_FLAGS = {"ebb_space.cu": ["-Xptxas", "-O1"], "ebb_flight.cu": ["-Xptxas", "-O1"]}
+# per source: further flags (ptxas's own -O3 is the fastest for every source: the flight ticks' shorter searches no longer
+# wait on instruction fetch, so the flight tick, 65,536 worlds of 4 ships, takes 347 us a tick with it and 369 with -O1,
+# the space layer's, 16,384 worlds a thread each, 1.48 and 1.55 ms)
+SOURCE_FLAGS: dict = {}
 
 
 def nvcc() -> str:

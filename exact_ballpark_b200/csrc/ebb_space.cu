@@ -21,12 +21,15 @@
 namespace ebb {
 namespace space {
 
+// a thread a world, `per_warp` of a warp's lanes (registers: 128, 4 blocks a multiprocessor; 80 ran 16,384 4-ship worlds
+// 2-4 % slower)
 template <bool WM>
-__global__ void __launch_bounds__(128, 6) tape_kernel(const __grid_constant__ EbbFlightState p,
+__global__ void __launch_bounds__(128, 4) tape_kernel(const __grid_constant__ EbbFlightState p,
                                                    const __grid_constant__ EbbSpaceState s,
-                                                   const __grid_constant__ EbbSpaceTape t) {
-    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= s.worlds) return;
+                                                   const __grid_constant__ EbbSpaceTape t, int per_warp) {
+    const int lane = (int)(threadIdx.x & 31);
+    const int64_t w = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp + lane;
+    if (lane >= per_warp || w >= s.worlds) return;
     run_tape<WM>(&p, &s, &t, w);
 }
 
@@ -133,11 +136,18 @@ int ebb_space_tape(const EbbFlightState* park, const EbbSpaceState* s, const Ebb
         else
             ebb::space::tape_kernel_warp<false><<<grid, 128, 0, st>>>(*park, *s, *t);
     } else {
-        const unsigned grid = (unsigned)((s->worlds + block - 1) / block);
+        // Worlds a warp: a warp's time grows with them (their programs diverge: 4 of 32 lanes busy), the worlds' own with the
+        // warps in flight (their states contend for the cache), so the worlds a warp rise with the square root of all of
+        // them: 2 at 256 worlds, 4 at 1,024, ... 32 from 65,536. Ticks of 4-ship worlds, ms, at 32 a warp and so: 256 worlds
+        // 0.94 and 0.36, 1,024 0.96 and 0.47, 4,096 1.03 and 0.65, 16,384 1.40 and 1.31 (8 a warp 1.40, 4 2.06).
+        int per = 2;
+        while (per < 32 && (int64_t)per * per * 64 < s->worlds) per *= 2;
+        const int64_t warps = (s->worlds + per - 1) / per;
+        const unsigned grid = (unsigned)((warps + block / 32 - 1) / (block / 32));
         if (s->pitch > 0)
-            ebb::space::tape_kernel<true><<<grid, block, 0, st>>>(*park, *s, *t);
+            ebb::space::tape_kernel<true><<<grid, block, 0, st>>>(*park, *s, *t, per);
         else
-            ebb::space::tape_kernel<false><<<grid, block, 0, st>>>(*park, *s, *t);
+            ebb::space::tape_kernel<false><<<grid, block, 0, st>>>(*park, *s, *t, per);
     }
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;
