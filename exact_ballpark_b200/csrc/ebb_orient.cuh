@@ -255,8 +255,10 @@ __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, co
                                             int* n1_out, F3* a1_out, float* k1_out) {
     const int lane = threadIdx.x & 31;
     const float* kept = found + FOUND_FLOATS + lane;
-    bool settled = true;
+    bool settled = true, near = false, pass1 = false;
     Bounds bd;
+    float first = 0.0f, foot = 0.0f, kb = 0.0f, k1 = 0.0f;
+    int n = 0;
     float o2 = 0.0f;
     bool plain = false;
     if ((want >> lane) & 1) {
@@ -271,26 +273,44 @@ __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, co
         settled = false;
         if (!plain) {
             const float l2 = __log2f(mine.tf), m2 = ROLL ? mine.max_alpha * mine.max_alpha : mine.limit2;
-            const float first = __fmaf_rn(-bd.A, mine.tf, bd.tau), foot = __fdividef(to, o2);
-            int below = 0, n = TORQUE_STEPS;
+            first = __fmaf_rn(-bd.A, mine.tf, bd.tau);
+            foot = __fdividef(to, o2);
+            int below = 0;
+            n = TORQUE_STEPS;
 #pragma unroll 1
             while (n - below > 1) {
                 const int mid = (below + n) >> 1;
                 const float nf = (float)mid, k = exp2_near(nf * l2), u = 1.0f - k;
                 const float num = __fmaf_rn(-bd.A, k, bd.tau), den = bd.tau * __fmaf_rn(-bd.A, u, nf * dt);
-                const float near = fminf(fmaxf(foot, first), num);   // (num's best up to there: so a pass stays one)
-                const bool pass = __fmaf_rn(__fmaf_rn(o2, near, -2.0f * to), near, t2) < m2 * den * den;
+                const float best = fminf(fmaxf(foot, first), num);   // (num's best up to there: so a pass stays one)
+                const bool pass = __fmaf_rn(__fmaf_rn(o2, best, -2.0f * to), best, t2) < m2 * den * den;
                 below = pass ? below : mid;
                 n = pass ? mid : n;
             }
-            const float kb = kappa_at(kept, n - 1, mine.tf);
+            kb = kappa_at(kept, n - 1, mine.tf);
             const bool none = n == TORQUE_STEPS;             // (then the 99th's values)
-            const float k1 = none ? kb : fmul(kb, mine.tf);
-            const bool pass = candidate<ROLL>(mine, k1, ndt_tab[none ? n - 1 : n], a1_out);
-            settled = (none ? !pass : pass) &&
+            k1 = none ? kb : fmul(kb, mine.tf);
+            pass1 = candidate<ROLL>(mine, k1, ndt_tab[none ? n - 1 : n], a1_out);
+            near = n < TORQUE_STEPS - 1;
+            settled = (none ? !pass1 : pass1) &&
                       (n == 1 || none_before<ROLL>(bd, mine, o2, first, foot, kb, n - 1, ndt_tab[n - 1], dt));
             *n1_out = n;
             *k1_out = k1;
+        }
+    }
+    if (!settled && near) {
+        const int q = pass1 ? n - 1 : n + 1;                 // (a passing guess of 1 is settled)
+        const float kq = pass1 ? kb : fmul(k1, mine.tf);
+        F3 a1;
+        const bool pass = candidate<ROLL>(mine, kq, ndt_tab[q], &a1);
+        const int m = pass1 ? n - 2 : n - 1;                 // the candidates not yet computed
+        settled = (pass1 || pass) &&
+                  (m == 0 || none_before<ROLL>(bd, mine, o2, first, foot, pass1 ? kappa_at(kept, m, mine.tf) : kb, m,
+                                               ndt_tab[m], dt));
+        if (pass) {
+            *a1_out = a1;
+            *n1_out = q;
+            *k1_out = kq;
         }
     }
     const unsigned open = __ballot_sync(FULL_WARP, !settled);
