@@ -14,9 +14,6 @@
 #ifndef EBB_SPACE_WARP_BLOCKS
 #define EBB_SPACE_WARP_BLOCKS 4
 #endif
-#ifndef EBB_SPACE_LAYERS_BLOCKS
-#define EBB_SPACE_LAYERS_BLOCKS 4
-#endif
 
 namespace ebb {
 namespace space {
@@ -47,8 +44,12 @@ __global__ void __launch_bounds__(128, EBB_SPACE_WARP_BLOCKS) tape_kernel_warp(c
 // Several layers' tapes in one launch, a warp a world (world-major): a batch's size classes one after another each held
 // about a tenth of the chip's warps until its slowest world was done (8,000 partition worlds, 269 blocks a class of 64 or
 // 128 slots); side by side the small classes fill the large one's gaps (6.4 -> 5.3 ms a tick). The layers' blocks follow in
-// the order given, so that the first layer's (the longest programs) start first. Blocks a multiprocessor, in ms a tick at
-// 8,000 and 24,000 worlds: 3 5.2 and 10.9, 4 5.3 and 10.5, 6 5.5 and 10.7, 8 5.6 and 10.7.
+// the order given, so that the first layer's (the longest programs) start first. BLOCKS a multiprocessor: while the batch
+// is a few waves the tick is its longest programs, which 255 registers (2 blocks) shorten; with more waves the blocks in
+// flight count, and 128 registers (4) win. Ms a tick at 2 and 4 blocks: 1,000 worlds of 1 to 128 ships 1.47 and 1.56, 4,000
+// 2.29 and 2.56, 8,000 3.52 and 3.94, 10,000 4.40 and 4.53, 11,000 4.84 and 4.80, 14,000 5.95 and 5.80, 24,000 10.0 and
+// 9.56 (3 blocks: 8,000 3.78, 24,000 9.80; 5: 4.04 and 9.67): the line is at 9 waves of the 2 (10,656 worlds).
+constexpr int64_t LONG_BLOCKS = 9 * 2 * 148;
 struct Layers {
     EbbSpaceState s[EBB_SPACE_MAX_LAYERS];
     EbbSpaceTape t[EBB_SPACE_MAX_LAYERS];
@@ -56,8 +57,9 @@ struct Layers {
     int count;
 };
 
-__global__ void __launch_bounds__(128, EBB_SPACE_LAYERS_BLOCKS) tape_kernel_layers(const __grid_constant__ EbbFlightState p,
-                                                                                  const __grid_constant__ Layers m) {
+template <int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) tape_kernel_layers(const __grid_constant__ EbbFlightState p,
+                                                                  const __grid_constant__ Layers m) {
     __shared__ Coop scratch[4];
     int l = 0;
     while (l + 1 < m.count && blockIdx.x >= m.first[l + 1]) ++l;
@@ -176,7 +178,10 @@ int ebb_space_tapes(const EbbFlightState* park, const EbbSpaceState* s, const Eb
     }
     if (m.count == 0) return 0;
     m.first[m.count] = (unsigned)blocks;
-    ebb::space::tape_kernel_layers<<<(unsigned)blocks, 128, 0, (cudaStream_t)stream>>>(*park, m);
+    if (blocks <= ebb::space::LONG_BLOCKS)
+        ebb::space::tape_kernel_layers<2><<<(unsigned)blocks, 128, 0, (cudaStream_t)stream>>>(*park, m);
+    else
+        ebb::space::tape_kernel_layers<4><<<(unsigned)blocks, 128, 0, (cudaStream_t)stream>>>(*park, m);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;
 }
