@@ -23,8 +23,8 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
               "-prec-div=true", "-prec-sqrt=true", "-ftz=false", "-Xcompiler", "-fPIC,-ffp-contract=off,-fno-fast-math",
               "-Xptxas", "-v", "-shared"]
 # per source: further flags (ptxas's own -O3 is the fastest for every source: the flight ticks' shorter searches no longer
-# wait on instruction fetch, so the flight tick, 65,536 worlds of 4 ships, takes 347 us a tick with it and 369 with -O1,
-# the space layer's, 16,384 worlds a thread each, 1.48 and 1.55 ms)
+# wait on instruction fetch, so the flight tick, 65,536 worlds of 4 ships, took 347 us a tick with it and 369 with -O1,
+# the space layer's, 16,384 worlds a thread each, 1.48 and 1.55 ms, as measured when the flag was taken out)
 SOURCE_FLAGS: dict = {}
 
 

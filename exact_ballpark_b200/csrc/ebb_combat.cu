@@ -37,7 +37,7 @@
 
 // Resident blocks a multiprocessor is asked to fit (the register budget the compiler gets), per tick: the combat tick
 // at 80 registers (3 blocks of 256 threads), the composed tick at 128 with its Gradient and commit out of line (2
-// blocks): measured fastest on B200 at 65,536 worlds (1.21 and 1.65 ms a tick, against 1.54 and 2.84 ms with the
+// blocks): measured fastest on B200 at 65,536 worlds, while the searches took a warp a ship (1.21 and 1.65 ms a tick, against 1.54 and 2.84 ms with the
 // composed tick at 80 registers, everything inlined and 128-thread blocks)
 #ifndef EBB_COMBAT_MIN_BLOCKS
 #define EBB_COMBAT_MIN_BLOCKS 3

@@ -9,10 +9,12 @@
 // the laws without their roundings, computes that candidate as the serial loop does (its kappa1 = tf^n1 by the serial
 // loop's own float products, every eighth of them kept), and shows that every candidate before it fails by one comparison
 // with bounds on what the serial loop's rounded operations can give (none_before). Where that does not settle a ship (one
-// in thirty), eight lanes walk its candidates, four ships at a time, each told by bounds without a division, only those
-// too near the maximum to be told computed (warp_walk). So the n1, alpha1 and kappa1 are the serial loop's, bit for bit.
-// A tick of 65,536 worlds of 4 ships: 369 us; with 32 lanes on one ship and block of 32 candidates, all computed, 584; by
-// the walk alone 636. The set-up, the braking rounds (logf, pow) and ApplyTorque are one lane a ship too.
+// search in ten) the neighbouring candidate is computed, which leaves 1 to 3 in 100: those overshoot, and the law passes
+// long after num's nearest. Eight lanes walk these ones' candidates, four ships at a time, each told by bounds without a
+// division, only those too near the maximum to be told computed (warp_walk). So the n1, alpha1 and kappa1 are the serial
+// loop's, bit for bit. A tick of 65,536 worlds of 4 ships: 286 us; without the neighbour 347; with 32 lanes on one ship and
+// block of 32 candidates, all computed, 584; by the walk alone 636 (the last two at -O1). A second bisection past num's
+// nearest in place of the walk 312, a scan of the law from there 401. The set-up, the braking rounds (logf, pow) and ApplyTorque are one lane a ship too.
 #pragma once
 
 #include "ebb_flight.cuh"
@@ -248,8 +250,8 @@ __device__ __forceinline__ bool none_before(const Bounds& q, const Quest& s, flo
 
 // The round's searches of the lanes in `want`: each searching lane's n1, kappa1 and alpha1. A lane guesses its own ship's
 // n1 by bisection on the laws without their roundings, num's best so far in place of num, so that a passing candidate is
-// followed by passing ones alone; computes that candidate as the serial loop does, and tells by bounds whether every one before it fails; the ships for
-// which the two don't settle it are walked.
+// followed by passing ones alone; computes that candidate as the serial loop does, and tells by bounds whether every one before it fails; where the two
+// don't settle it, the one before a guess that passes or after one that fails is computed, and the ships still open walked.
 template <bool ROLL>
 __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, const float* ndt_tab, float* found, float dt,
                                             int* n1_out, F3* a1_out, float* k1_out) {

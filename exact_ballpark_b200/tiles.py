@@ -102,9 +102,9 @@ def shape_for(rows: int, max_world: int) -> tuple:
     with its ships (their modes, their searches, the slowest of them), so few rows are spread over the chip, 4 to 32 a
     warp, until each of its schedulers has a warp; more rows take full warps, in blocks of 128 threads (their ends even
     out over the multiprocessors) until a wave of 256-thread blocks is full (their warps share the instruction cache).
-    Dynamical orientation on, us a tick, as 256-row tiles and so: 64 worlds of 4 ships 64 and 52, 600 72 and 62, 2,000 73
-    and 67, 5,000 77 and 74, 20,000 115 and 105, 65,536 344 and 344 (128-thread blocks: 367); 100 worlds of 1 to 128 ships
-    75 and 69. Without it every shape of 64 worlds takes 14."""
+    Dynamical orientation on, us a tick, as 256-row tiles and so: 64 worlds of 4 ships 50 and 43, 600 58 and 53, 2,000 61
+    and 57, 5,000 64 and 62, 20,000 92 and 85, 65,536 264 and 264 (128-thread blocks: 282); 100 worlds of 1 to 128 ships
+    61 and 59. Without it every shape of 64 worlds takes 14."""
     warp = 4
     while warp < 32 and rows > warp * SPREAD_WARPS:
         warp *= 2
