@@ -20,6 +20,7 @@
 
 #include "../../include/ebb.h"
 #include "ebb_arith.cuh"
+#include "ebb_launch.cuh"
 #include "ebb_libm.cuh"
 
 namespace ebb {
@@ -1074,10 +1075,8 @@ int ebb_collide_tick(const EbbCollideState* s, const uint8_t* active, int32_t* s
     const auto kernel = s->statics > 0                        ? ebb::collide::tick_kernel<true, ebb::collide::BLOCKS_STATICS>
                         : smem > ebb::collide::CROWDED_BYTES ? ebb::collide::tick_kernel<false, ebb::collide::BLOCKS_CROWDED>
                                                              : ebb::collide::tick_kernel<false, ebb::collide::BLOCKS_BALLS>;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
+    const cudaError_t allowed = ebb::allow_shared(kernel, smem);
+    if (allowed != cudaSuccess) return (int)allowed;
     kernel<<<grid, threads, smem, (cudaStream_t)stream>>>(*s, active, status);
     return launched();
 }

@@ -32,6 +32,7 @@
 
 #include "../../include/ebb.h"
 #include "ebb_flight.cuh"
+#include "ebb_launch.cuh"
 #include "ebb_orient.cuh"
 #include "ebb_rows.cuh"
 
@@ -1058,10 +1059,8 @@ int launch_tick(const EbbComposedState& x, bool collide, const int64_t* tile_row
         return EBB_EINVAL;
     const size_t smem = ebb::combat::tick_smem_bytes(block, collide);
     auto kernel = collide ? ebb::combat::tick_kernel<true> : ebb::combat::tick_kernel<false>;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
+    const cudaError_t allowed = ebb::allow_shared(kernel, smem);
+    if (allowed != cudaSuccess) return (int)allowed;
     kernel<<<(unsigned)tiles, block, smem, (cudaStream_t)stream>>>(x, tile_rows, tiles, status);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;

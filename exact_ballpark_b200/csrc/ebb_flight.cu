@@ -20,6 +20,7 @@
 
 #include "../../include/ebb.h"
 #include "ebb_flight.cuh"
+#include "ebb_launch.cuh"
 #include "ebb_orient.cuh"
 #include "ebb_rows.cuh"
 
@@ -801,10 +802,8 @@ int ebb_flight_tick_tiled(const EbbFlightState* s, const int64_t* tile_rows, int
     const size_t smem = ebb::flight::tiled_smem_bytes(tile_cap, block);
     auto kernel = (tile_cap <= block && grid >= tiles) ? ebb::flight::tiled_kernel<true>
                                                          : ebb::flight::tiled_kernel<false>;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
+    const cudaError_t allowed = ebb::allow_shared(kernel, smem);
+    if (allowed != cudaSuccess) return (int)allowed;
     kernel<<<(unsigned)grid, block, smem, (cudaStream_t)stream>>>(*s, tile_rows, tiles, tile_cap, status);
     return launched();
 }
@@ -819,10 +818,8 @@ int ebb_flight_tick_worlds(const EbbFlightState* s, const int64_t* worlds, const
     const size_t smem = ebb::flight::listed_smem_bytes(tile_cap, block);
     auto kernel = (tile_cap <= block && grid >= tiles) ? ebb::flight::worlds_kernel<true>
                                                          : ebb::flight::worlds_kernel<false>;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
+    const cudaError_t allowed = ebb::allow_shared(kernel, smem);
+    if (allowed != cudaSuccess) return (int)allowed;
     kernel<<<(unsigned)grid, block, smem, (cudaStream_t)stream>>>(*s, worlds, tile_worlds, tiles, tile_cap, active,
                                                                   status);
     return launched();
