@@ -3,18 +3,23 @@
 // GotoTorqueBreaks full.py:2155, GotoRollBreaks full.py:2224, ApplyTorque full.py:2292), warp-cooperative.
 //
 // Each torque search tries n1 = 1, 2, ... 99 accelerating ticks and keeps the first whose torque is within the
-// maximum, in up to five rounds (each round re-derives the braking ticks n2): seven searches a ship and tick on the
-// flight benchmark's worlds, their n1 a median of 10 and a mean of 16. What bounds it is the issue of instructions, so the
-// searches avoid most candidates, and every lane searches for its own ship (warp_search): it guesses n1 by bisection on
-// the laws without their roundings, computes that candidate as the serial loop does (its kappa1 = tf^n1 by the serial
-// loop's own float products, every eighth of them kept), and shows that every candidate before it fails by one comparison
-// with bounds on what the serial loop's rounded operations can give (none_before). Where that does not settle a ship (one
-// search in ten) the neighbouring candidate is computed, which leaves 1 to 3 in 100: those overshoot, and the law passes
-// long after num's nearest. Eight lanes walk these ones' candidates, four ships at a time, each told by bounds without a
-// division, only those too near the maximum to be told computed (warp_walk). So the n1, alpha1 and kappa1 are the serial
-// loop's, bit for bit. A tick of 65,536 worlds of 4 ships: 286 us; without the neighbour 347; with 32 lanes on one ship and
-// block of 32 candidates, all computed, 584; by the walk alone 636 (the last two at -O1). A second bisection past num's
-// nearest in place of the walk 312, a scan of the law from there 401. The set-up, the braking rounds (logf, pow) and ApplyTorque are one lane a ship too.
+// maximum, in up to five rounds (each round re-derives the braking ticks n2): seven searches a ship and tick in the first
+// ticks of the flight benchmark's worlds (their n1 a median of 10 and a mean of 16), 2.4 by the 200th. What bounds it is
+// the issue of instructions, so the searches avoid most candidates, and every lane searches for its own ship
+// (warp_search): it guesses n1 by bisection on the laws without their roundings, computes that candidate as the serial
+// loop does (its kappa1 = tf^n1 by the serial loop's own float products, every eighth of them kept), and shows that every
+// candidate before it fails by one comparison with bounds on what the serial loop's rounded operations can give
+// (none_before). Where that does not settle a ship the neighbouring candidate is computed. What is left overshoots: the law
+// passes long after num's nearest (the rolls at a mean n1 of 13 in the first ticks, 38 to 44 late in a flight). Eight lanes
+// walk these ones' candidates, four ships at a time, from the last one shown to fail (of 96 to 99 in 100 every one up to
+// the guess is), each told by bounds without a division, only those too near the maximum to be told computed (warp_walk).
+// So the n1, alpha1 and kappa1 are the serial loop's, bit for bit.
+// Of the searches 1 in 100 are walked at the 4th tick from rest, 14 at the 16th, 22 and 25 at the 32nd and 64th, 19 at the
+// 128th and 200th. 65,536 worlds of 4 ships, us a tick at the 4th, 16th, 64th and 200th: 216, 313, 383 and 369; walked from
+// the first candidate on 224, 344, 438 and 437; with 32 lanes on one ship and block of 32 candidates, all computed, 570,
+// 506, 410 and 417. Over the first 8 ticks a second bisection past num's nearest in place of the walk was slower (312 us
+// and 286), so were a scan of the law from there (401), the walk alone (636) and no neighbour (347). The set-up, the
+// braking rounds (logf, pow) and ApplyTorque are one lane a ship too.
 #pragma once
 
 #include "ebb_flight.cuh"
@@ -118,10 +123,12 @@ __device__ __forceinline__ bool candidate(const Quest& s, float k1, float n1dt, 
 }
 
 // The searches of the lanes in `want` candidate by candidate, four ships at a time, eight lanes a ship: each lane's n1 and
-// kappa1 (n1 = 100 with the 99th candidate's kappa1 when none passes), and its alpha1, left in that lane
+// kappa1 (n1 = 100 with the 99th candidate's kappa1 when none passes), and its alpha1, left in that lane. `fail`: every
+// candidate up to it is known to fail, so a ship's walk starts with the block of GROUP that holds the next one.
 template <bool ROLL>
 __device__ __forceinline__ void warp_walk(unsigned want, const Quest& mine, const Bounds& mine_bd, float o2, bool plain,
-                                          const float* ndt_tab, float* found, int* n1_out, F3* a1_out, float* k1_out) {
+                                          int fail, const float* ndt_tab, float* found, int* n1_out, F3* a1_out,
+                                          float* k1_out) {
     const int lane = threadIdx.x & 31, sub = lane & (GROUP - 1), first = lane & ~(GROUP - 1);
     const unsigned group = ((1u << GROUP) - 1u) << first;
     const bool searching = (want >> lane) & 1;
@@ -153,19 +160,21 @@ __device__ __forceinline__ void warp_walk(unsigned want, const Quest& mine, cons
             omega2 = wbc(o2, from);
         }
         const bool untold = wbc((int)plain, from) != 0;
-        float k1 = tf;                                       // kappa_{sub + 1}
+        const int failed = wbc(fail, from);
+        int b = failed & ~(GROUP - 1);
+        float k1 = b ? fmul(found[FOUND_FLOATS + (b / GROUP - 1) * 32 + from], tf) : tf;
 #pragma unroll
-        for (int i = 1; i < GROUP; ++i)
+        for (int i = 1; i < GROUP; ++i)                      // kappa_{b + sub + 1}
             if (i <= sub) k1 = fmul(k1, tf);
         bool open = src >= 0;
-        for (int b = 0;; b += GROUP) {
+        for (;; b += GROUP) {
             const int n = b + sub + 1;
             const float n1dt = ndt_tab[n < TORQUE_STEPS ? n : TORQUE_STEPS - 1];
             int told = 0;
             if (!untold)
                 told = ROLL ? tell_roll(bd, target.x, omega0.x, max_alpha, k1, n1dt)
                             : tell_heading(bd, target, omega0, omega2, limit2, k1, n1dt);
-            if (n >= TORQUE_STEPS) told = -1;
+            if (n >= TORQUE_STEPS || n <= failed) told = -1;
             unsigned maybe = __ballot_sync(FULL_WARP, open && told >= 0) & group;
             const bool doubt = maybe != 0 && lane == __ffs(maybe) - 1 && told == 0;
             if (__any_sync(FULL_WARP, doubt)) {              // a group's first is not told: its candidates are computed
@@ -226,8 +235,8 @@ __device__ __forceinline__ float kappa_at(const float* kept, int n, float tf) {
     return k;
 }
 // Whether every candidate 1 .. n fails, told at once: num rises with n (kappa1 falls) from `first`, so the least
-// |target - omega0 num| is at num's nearest to the line's foot (the same roll: where the coast ends on the target); den rises with n but for what the kappas' own rounding takes back, at most
-// |A| (1 - tf + 2^-23) - dt a candidate.
+// |target - omega0 num| is at num's nearest to the line's foot (the same roll: where the coast ends on the target); den
+// rises with n but for what the kappas' own rounding takes back, at most |A| (1 - tf + 2^-23) - dt a candidate.
 template <bool ROLL>
 __device__ __forceinline__ bool none_before(const Bounds& q, const Quest& s, float o2, float first, float foot, float kn,
                                             int n, float ndt_n, float dt) {
@@ -250,8 +259,9 @@ __device__ __forceinline__ bool none_before(const Bounds& q, const Quest& s, flo
 
 // The round's searches of the lanes in `want`: each searching lane's n1, kappa1 and alpha1. A lane guesses its own ship's
 // n1 by bisection on the laws without their roundings, num's best so far in place of num, so that a passing candidate is
-// followed by passing ones alone; computes that candidate as the serial loop does, and tells by bounds whether every one before it fails; where the two
-// don't settle it, the one before a guess that passes or after one that fails is computed, and the ships still open walked.
+// followed by passing ones alone; computes that candidate as the serial loop does, and tells by bounds whether every one
+// before it fails; where the two don't settle it, the one before a guess that passes or after one that fails is computed,
+// and the ships still open walked from what was shown to fail.
 template <bool ROLL>
 __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, const float* ndt_tab, float* found, float dt,
                                             int* n1_out, F3* a1_out, float* k1_out) {
@@ -260,7 +270,7 @@ __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, co
     bool settled = true, near = false, pass1 = false;
     Bounds bd;
     float first = 0.0f, foot = 0.0f, kb = 0.0f, k1 = 0.0f;
-    int n = 0;
+    int n = 0, fail = 0;                                     // every candidate up to `fail` fails
     float o2 = 0.0f;
     bool plain = false;
     if ((want >> lane) & 1) {
@@ -294,8 +304,8 @@ __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, co
             k1 = none ? kb : fmul(kb, mine.tf);
             pass1 = candidate<ROLL>(mine, k1, ndt_tab[none ? n - 1 : n], a1_out);
             near = n < TORQUE_STEPS - 1;
-            settled = (none ? !pass1 : pass1) &&
-                      (n == 1 || none_before<ROLL>(bd, mine, o2, first, foot, kb, n - 1, ndt_tab[n - 1], dt));
+            if (n > 1 && none_before<ROLL>(bd, mine, o2, first, foot, kb, n - 1, ndt_tab[n - 1], dt)) fail = n - 1;
+            settled = (none ? !pass1 : pass1) && fail == n - 1;
             *n1_out = n;
             *k1_out = k1;
         }
@@ -305,10 +315,14 @@ __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, co
         const float kq = pass1 ? kb : fmul(k1, mine.tf);
         F3 a1;
         const bool pass = candidate<ROLL>(mine, kq, ndt_tab[q], &a1);
-        const int m = pass1 ? n - 2 : n - 1;                 // the candidates not yet computed
-        settled = (pass1 || pass) &&
-                  (m == 0 || none_before<ROLL>(bd, mine, o2, first, foot, pass1 ? kappa_at(kept, m, mine.tf) : kb, m,
-                                               ndt_tab[m], dt));
+        if (pass1) {                                         // the candidates before the one before
+            const int m = n - 2;
+            settled = m == 0 || none_before<ROLL>(bd, mine, o2, first, foot, kappa_at(kept, m, mine.tf), m, ndt_tab[m], dt);
+            fail = settled ? m : 0;
+        } else if (fail == n - 1) {
+            settled = pass;
+            fail = q;                                        // (or it passes)
+        }
         if (pass) {
             *a1_out = a1;
             *n1_out = q;
@@ -316,7 +330,7 @@ __device__ __forceinline__ void warp_search(unsigned want, const Quest& mine, co
         }
     }
     const unsigned open = __ballot_sync(FULL_WARP, !settled);
-    if (open) warp_walk<ROLL>(open, mine, bd, o2, plain, ndt_tab, found, n1_out, a1_out, k1_out);
+    if (open) warp_walk<ROLL>(open, mine, bd, o2, plain, fail, ndt_tab, found, n1_out, a1_out, k1_out);
 }
 
 // The warp's orientation step: every lane calls it together (lanes whose ship is off pass through). `found` is the
