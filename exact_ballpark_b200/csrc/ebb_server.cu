@@ -327,11 +327,43 @@ __device__ int64_t loc_of(const EbbServerState& s, int32_t kind, bool tested, in
     return !tested && kind == EBB_KIND_CLOAK ? (s.settled[row < 0 ? 0 : row] ? 0 : -1) : loc_in;
 }
 
-// The queue pass by a world's only lane (worlds of at most IDS_IN_REGISTERS rows): each push's rows, CloakBall's bubble and
-// the duplicate test, nothing written to the park (so the loads of later slots need not wait for earlier slots'
-// commands); the world's ids held in registers for the lookups.
+// Whether the world's listed balls are ids 1, 2, ... in order up to its last (a ball's row is then at its id's position,
+// and an id outside them is no ball's), and one past the last listed
+template <int G>
+__device__ bool ids_in_order(const World& x, const Group<G>& g, int64_t* span_out) {
+    int64_t span = 0;
+    bool ordered = true;
+    if constexpr (G == 1) {
+        for (int64_t k = 0; k < x.s.width; ++k) {
+            if (x.rows[k] < 0) continue;
+            ordered = ordered && span == k && x.ids[k] == k + 1;
+            span = k + 1;
+        }
+    }
+    for (int64_t k0 = 0; G > 1 && k0 < x.s.width; k0 += G) {
+        const int64_t k = k0 + g.sub;
+        const bool listed = g.on && k < x.s.width && x.rows[k] >= 0;
+        const bool fits = !g.on || k >= x.s.width || (listed ? x.ids[k] == k + 1 : true);
+        const unsigned m = __ballot_sync(0xffffffffu, listed) & g.mask;
+        if (m) {
+            // the positions up to this chunk's last listed ball all listed, and the chunk follows the one before
+            const int at = 31 - __clz(m);
+            const unsigned want = g.mask & ((2u << at) - 1u);
+            if (m != want || span != k0) ordered = false;
+            span = k0 + (at - g.first) + 1;
+        }
+        ordered = g.all(fits) && ordered;
+    }
+    *span_out = span;
+    return ordered;
+}
+
+// The queue pass by a world's only lane: each push's rows, CloakBall's bubble and the duplicate test, nothing written to
+// the park (so the loads of later slots need not wait for earlier slots' commands); the ids of a world of at most
+// IDS_IN_REGISTERS rows held in registers for the lookups (WIDE: a world of more).
 constexpr int IDS_IN_REGISTERS = 8;
 
+template <bool WIDE>
 __device__ void queue_alone(const World& x, const EbbServerQueue& q) {
     const EbbServerState& s = x.s;
     const int64_t W = s.worlds, w = x.w, J = q.slots;
@@ -349,10 +381,14 @@ __device__ void queue_alone(const World& x, const EbbServerQueue& q) {
     int64_t ids[IDS_IN_REGISTERS], rows[IDS_IN_REGISTERS];
 #pragma unroll
     for (int k = 0; k < IDS_IN_REGISTERS; ++k) {
-        ids[k] = k < s.width ? x.ids[k] : 0;
-        rows[k] = k < s.width ? x.rows[k] : -1;
+        ids[k] = !WIDE && k < s.width ? x.ids[k] : 0;
+        rows[k] = !WIDE && k < s.width ? x.rows[k] : -1;
     }
+    int64_t span = 0;
+    const bool ordered = WIDE && ids_in_order(x, Group<1>(true), &span);
     auto lookup = [&](int64_t id) -> int64_t {
+        if (ordered) return id >= 1 && id <= span ? x.rows[id - 1] : -1;
+        if (WIDE) return x.lookup(id, span);
         int64_t found = -1;
 #pragma unroll
         for (int k = IDS_IN_REGISTERS - 1; k >= 0; --k)       // the first match wins
@@ -403,28 +439,11 @@ __device__ void queue_alone(const World& x, const EbbServerQueue& q) {
     }
 }
 
-// Whether the world's listed balls are ids 1, 2, ... in order up to its last (a ball's row is then at its id's position,
-// and an id outside them is no ball's), and one past the last listed
-template <int G>
-__device__ bool ids_in_order(const World& x, const Group<G>& g, int64_t* span_out) {
-    int64_t span = 0;
-    bool ordered = true;
-    for (int64_t k0 = 0; k0 < x.s.width; k0 += G) {
-        const int64_t k = k0 + g.sub;
-        const bool listed = g.on && k < x.s.width && x.rows[k] >= 0;
-        const bool fits = !g.on || k >= x.s.width || (listed ? x.ids[k] == k + 1 : true);
-        const unsigned m = __ballot_sync(0xffffffffu, listed) & g.mask;
-        if (m) {
-            // the positions up to this chunk's last listed ball all listed, and the chunk follows the one before
-            const int at = 31 - __clz(m);
-            const unsigned want = g.mask & ((2u << at) - 1u);
-            if (m != want || span != k0) ordered = false;
-            span = k0 + (at - g.first) + 1;
-        }
-        ordered = g.all(fits) && ordered;
-    }
-    *span_out = span;
-    return ordered;
+__device__ void queue_alone(const World& x, const EbbServerQueue& q) {
+    if (x.s.width <= IDS_IN_REGISTERS)
+        queue_alone<false>(x, q);
+    else
+        queue_alone<true>(x, q);
 }
 
 // The queue pass: each push's rows, CloakBall's bubble and the duplicate test; nothing written to the park. Returns whether
@@ -671,15 +690,24 @@ __global__ void __launch_bounds__(128, 4) server_kernel(const __grid_constant__ 
     }
 }
 
-// The lanes a world, from its queue's slots and its rows, the `most` of the two. One when there are worlds enough to keep
-// the chip's warps in flight a thread each (a thread's accesses then coalesce with its neighbours', and nothing is voted
-// on); else enough for the slots and rows at once, up to a warp (a larger queue or world is taken 32 at a time). Pre-tick
-// and flags of 4-ship worlds (8 slots), us, one lane and eight: 8,192 worlds 22.9 and 15.9; 16,384 21.9 and 21.5; 24,576
-// 24.2 and 23.6; 32,768 25.7 and 31.2; 65,536 30.4 and 56.2. One ship (2 slots), 24,576 worlds: 9.8 and 20.5 (four lanes,
-// 65,536 worlds: 11.3 and 33.9). 8,000 worlds of 1 to 128 ships (256 slots): 1,436 us and, a warp a world, 140.
+// The lanes a world, from the worlds, their queues' slots and their rows: one when there are worlds enough to keep the chip's
+// warps in flight a thread each (a thread's accesses then coalesce with its neighbours', where a group's lanes read a slot
+// each, a sector or two apart for every world), else enough for the slots and rows at once, up to a warp (a larger queue or
+// world is taken 32 at a time). A lane a world is a chain over its slots and rows, which takes as long for one world as for
+// thousands; groups take the longer the more warps they fill: so the line rises with the rows, and with the rounds of a
+// queue longer than a warp. It lies where the two cost the same (a server tick with its park's, us, one lane and a group):
+// rows, slots 2, 16: 4,096 worlds 45 and 41, 6,144 43 and 63; 4, 8: 12,288 29 and 24, 24,576 37 and 38; 5, 10: 4,096 37 and
+// 34, 8,192 37 and 48, 65,536 88 and 298; 16, 16: 12,288 87 and 84, 24,576 135 and 173; 4, 32: 2,048 78 and 54, 4,096 80 and
+// 89, 65,536 199 and 1,181; 9, 18: 3,072 62 and 53, 4,096 64 and 72; 32, 4: 8,192 85 and 70, 16,384 114 and 143; 32, 64:
+// 32,768 499 and 471, 49,152 587 and 709; 128, 256: 16,384 1,741 and 876.
 enum class Lanes { one, four, eight, half, warp };
-inline Lanes lanes(int64_t worlds, int64_t most) {
-    if (most <= IDS_IN_REGISTERS && worlds > 2048 * most) return Lanes::one;
+inline Lanes lanes(int64_t worlds, int64_t slots, int64_t width) {
+    const int64_t most = slots > width ? slots : width, rows = width < 4096 ? width : 4096;
+    const int64_t line = most <= 8    ? 2048 * most
+                         : most <= 16 ? 4096 + 32 * rows * rows
+                         : slots <= 32 ? 2048 + 224 * rows
+                                       : (2048 + 224 * rows) * (64 + slots) / 32;
+    if (worlds > line) return Lanes::one;
     return most <= 4 ? Lanes::four : most <= 8 ? Lanes::eight : most <= 16 ? Lanes::half : Lanes::warp;
 }
 template <int G>
@@ -718,7 +746,7 @@ int ebb_server_tick(const EbbServerState* s, const EbbServerQueue* q, int phase,
          q->loc == nullptr || q->route == nullptr || q->notice == nullptr))
         return EBB_EINVAL;
     const cudaStream_t st = (cudaStream_t)stream;
-    const ebb::server::Lanes g = ebb::server::lanes(s->worlds, q->slots > s->width ? q->slots : s->width);
+    const ebb::server::Lanes g = ebb::server::lanes(s->worlds, q->slots, s->width);
     const cudaError_t e = g == ebb::server::Lanes::one     ? ebb::server::launch<1>(*s, *q, phase, j0, j1, st, block)
                           : g == ebb::server::Lanes::four  ? ebb::server::launch<4>(*s, *q, phase, j0, j1, st, block)
                           : g == ebb::server::Lanes::eight ? ebb::server::launch<8>(*s, *q, phase, j0, j1, st, block)
