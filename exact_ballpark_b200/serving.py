@@ -41,7 +41,7 @@ import torch
 
 from . import _native
 from .modes import _STATE_FIELD, _STORAGE, VecModesPark
-from .tiles import shape_for
+from .tiles import DEFAULT_BLOCK, DEFAULT_CAP, shape_for
 from .workloads import FlightWorlds, PackedWorlds, flight_worlds, ragged_ships
 
 STATE_BYTES_PER_ROW = sum((8 if dt in (torch.float64, torch.int64) else 4 if dt in (torch.float32, torch.int32) else 1)
@@ -323,18 +323,22 @@ class Staged:
 
 class Server:
     """The continuous-batching loop (module docstring). `budget_bytes` of device state caps the resident rows
-    (ROW_BYTES a row; `rows` overrides it); `tile_cap` rows a tile of the listed-worlds tick, at least the largest
-    episode; `stage_rows` caps the rows staged ahead of admission, `stage_batch` the rows of one staging park; `depth`
-    steps may be in flight on the device; `keep` keeps each finished episode's final state in `results`. Staging runs
-    on a thread of its own (`close()` ends it)."""
+    (ROW_BYTES a row; `rows` overrides it); the listed-worlds tick takes tiles of `tile_cap` rows (at least the largest
+    episode) in blocks of `block` threads, `grid` of them, when any of the three is given (256 for a tile or a block left
+    out), else tiles and blocks as the live rows ask for (tiles.shape_for), up to 256; `stage_rows` caps the rows staged
+    ahead of admission, `stage_batch` the rows of one staging park; `depth` steps may be in flight on the device; `keep`
+    keeps each finished episode's final state in `results`. Staging runs on a thread of its own (`close()` ends it)."""
 
     def __init__(self, budget_bytes: float = 80e9, rows: int | None = None, dynamical: bool = True,
-                 new_orbit: bool = True, tile_cap: int = 256, block: int = 256, grid: int | None = None,
-                 device="cuda", keep: bool = True, max_ships: int = 256, stage_rows: int | None = None,
-                 stage_batch: int = 8192, depth: int = 1):
+                 new_orbit: bool = True, tile_cap: int | None = None, block: int | None = None,
+                 grid: int | None = None, device="cuda", keep: bool = True, max_ships: int = 256,
+                 stage_rows: int | None = None, stage_batch: int = 8192, depth: int = 1):
         capacity = int(rows) if rows is not None else int(budget_bytes // ROW_BYTES)
         if capacity <= 0:
             raise ValueError("the state budget holds no row")
+        self.by_rows = tile_cap is None and block is None and grid is None    # the tick's shape follows the live rows
+        tile_cap = DEFAULT_CAP if tile_cap is None else tile_cap
+        block = DEFAULT_BLOCK if block is None else block
         if max_ships > tile_cap:
             raise ValueError("an episode must fit one tile")
         self.park = VecModesPark(capacity, device=device, dynamical_orientation=dynamical, use_new_orbit=new_orbit)
@@ -468,9 +472,9 @@ class Server:
         main = torch.cuda.current_stream(self.dev)
         wb, tb = self.up_worlds.buffer(2 * c), self.up_tiles.buffer(c + 1)
         cap, block = self.tile_cap, self.block
-        if c:                                             # tiles and blocks no larger than the live rows ask for
+        if c and self.by_rows and self.grid is None:      # tiles and blocks no larger than the live rows ask for
             small, threads = shape_for(self.live_rows, int(self.table.len[:c].max()))
-            if small <= cap and self.grid is None:
+            if small <= cap:
                 cap, block = small, min(block, threads)
         worlds, tile_worlds = plan_worlds(self.table.start[:c], self.table.len[:c], cap, wb, tb)
         self._plan = (self.up_worlds.send(len(worlds), main), self.up_tiles.send(len(tile_worlds), main),
