@@ -38,8 +38,9 @@
 
 // Resident blocks a multiprocessor is asked to fit (the register budget the compiler gets), per tick: the combat tick
 // at 80 registers (3 blocks of 256 threads), the composed tick at 128 with its Gradient and commit out of line (2
-// blocks): measured fastest on B200 at 65,536 worlds, while the searches took a warp a ship (1.21 and 1.65 ms a tick, against 1.54 and 2.84 ms with the
-// composed tick at 80 registers, everything inlined and 128-thread blocks)
+// blocks). us a tick at the 64th tick, combat worlds of 8 and composed worlds of 9 at 2, 3 and 4 blocks (composed 1, 2 and
+// 3): 65,536 worlds 1,069, 984 and 983 (composed 1,773, 1,322 and 1,669); 16,384 worlds 219, 260 and 219 (444, 314 and 364);
+// 1,024 worlds 84, 88 and 94 (104, 105 and 113).
 #ifndef EBB_COMBAT_MIN_BLOCKS
 #define EBB_COMBAT_MIN_BLOCKS 3
 #endif

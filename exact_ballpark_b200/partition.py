@@ -252,8 +252,8 @@ def tune_partition(pw, dev, warm: int = 1, ticks: int = 2, arrangements=ARRANGEM
     runs it: the worlds are loaded, their sensors added, the server layer on top (the pilots' commands every tick, so
     the ships move as in the benchmark), `warm` ticks run, then `ticks` ticks each with every class's re-filings and
     HandleProximities timed alone (CUDA events); every arrangement starts from the same state and does the same work
-    (its results are bit-identical). The classes run one after another in a tick, so each takes its fastest
-    arrangement. Returns (plan {class: (lanes, block)}, {arrangement: {class: ms a tick}})."""
+    (its results are bit-identical). Each class takes the arrangement that is fastest alone: what the classes that run a
+    warp a world gain in a tick from their joint launch (space.tick_op) is not measured. Returns (plan {class: (lanes, block)}, {arrangement: {class: ms a tick}})."""
     times = {}
     for lanes, block in arrangements:
         plan = {cap: (lanes, block) for cap in CLASSES}

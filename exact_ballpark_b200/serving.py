@@ -126,7 +126,8 @@ class Rows:
     """Rows of park state in the park's device layout with no park behind them (finished episodes' final states): the
     storage tensors `_<name>`, `field()` in the reference layout, and `state()` for the native calls. The fields share one
     buffer, each from a 256-byte boundary, and a field's tensor is made when it is first asked for: a retirement makes one
-    allocation where a tensor a field made 34 (half of the loop's host time when every step retires something)."""
+    allocation where a tensor a field made 34 (256 episodes 46 -> 42 ms, 64 short ones 18 -> 16, with every step retiring
+    something). So a field kept keeps its whole retirement's rows: clone it to keep it alone."""
 
     def __init__(self, n: int, like: VecModesPark):
         self.n, self.dev = int(n), like.dev
@@ -286,6 +287,7 @@ class Result:
     ticks: int
 
     def field(self, name: str) -> torch.Tensor:
+        """The episode's rows of a field: a view of its retirement's buffer (`.clone()` to keep it without the rest)."""
         return self.rows.field(name, self.start, self.n)
 
 

@@ -102,9 +102,10 @@ def shape_for(rows: int, max_world: int) -> tuple:
     with its ships (their modes, their searches, the slowest of them), so few rows are spread over the chip, 4 to 32 a
     warp, until each of its schedulers has a warp; more rows take full warps, in blocks of 128 threads (their ends even
     out over the multiprocessors) until a wave of 256-thread blocks is full (their warps share the instruction cache).
-    Dynamical orientation on, us a tick, as 256-row tiles and so: 64 worlds of 4 ships 50 and 43, 600 58 and 53, 2,000 61
-    and 57, 5,000 64 and 62, 20,000 92 and 85, 65,536 264 and 264 (128-thread blocks: 282); 100 worlds of 1 to 128 ships
-    61 and 59. Without it every shape of 64 worlds takes 14."""
+    Dynamical orientation on, us a tick at the 8th tick from rest and at the 64th, as 256-row tiles and so: 64 worlds of 4
+    ships 56 64 and 46 56, 600 58 74 and 52 60, 2,000 60 78 and 58 69, 5,000 62 84 and 60 79, 20,000 89 126 and 85 116,
+    65,536 the same shape 285 383 (128-thread blocks: 311 417); 100 worlds of 1 to 128 ships 59 74 and 55 64. Without it
+    every shape of 64 worlds takes 14."""
     warp = 4
     while warp < 32 and rows > warp * SPREAD_WARPS:
         warp *= 2
