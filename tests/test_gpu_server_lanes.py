@@ -6,10 +6,25 @@ import numpy as np
 import pytest
 import torch
 
-from golden_util import bit_equal
 from test_gpu_server_groups import _calls, _run
 
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")]
+
+
+def same_bits(a, b) -> bool:
+    """The same bits, or both NaN; integers and flags in their own type (no way through a double)."""
+    if not a.dtype.is_floating_point:
+        return torch.equal(a, b)
+    bits = torch.int64 if a.dtype == torch.float64 else torch.int32
+    return bool(((a.contiguous().view(bits) == b.contiguous().view(bits)) | (a.isnan() & b.isnan())).all())
+
+
+def test_the_comparison_tells_bits_apart():
+    one = torch.tensor([2 ** 62 + 1, 5])
+    assert same_bits(one, one.clone()) and not same_bits(one, one - 1)
+    z = torch.tensor([0.0, float("nan")])
+    assert same_bits(z, z.clone()) and not same_bits(z, torch.tensor([-0.0, float("nan")]))
+    assert not same_bits(z, torch.tensor([0.0, 0.0]))
 
 
 @pytest.mark.parametrize("worlds,ships,shuffled,count", [(7000, 9, False, 4), (7000, 9, True, 4), (5000, 4, True, 11)])
@@ -20,7 +35,21 @@ def test_a_lane_a_world_matches_a_group(worlds, ships, shuffled, count):
     got = _run(worlds, ships, shuffled, calls, pads.tolist())
     assert len(got) == len(want)
     for i, (a, b) in enumerate(zip(want, got)):
-        assert a.dtype == b.dtype and bit_equal(a.cpu().numpy(), b.cpu().numpy()).all(), i
+        assert a.dtype == b.dtype and same_bits(a, b), i
+
+
+@pytest.mark.parametrize("worlds,ships,shuffled,count", [(37, 1, False, 3), (61, 4, True, 4), (19, 33, True, 9),
+                                                         (11, 130, False, 12)])
+def test_every_group_matches_by_bits(worlds, ships, shuffled, count):
+    calls = _calls(worlds, ships, count, 3)               # (the calls' values hold NaN, -0.0 and warps' 64-bit patterns)
+    want = _run(worlds, ships, shuffled, calls, [0] * (count + 1))
+    for total in (8, 16, 33, 70):
+        if total <= count:
+            continue
+        pads = np.bincount(np.random.default_rng(total).integers(0, count + 1, total - count), minlength=count + 1)
+        got = _run(worlds, ships, shuffled, calls, pads.tolist())
+        for i, (a, b) in enumerate(zip(want, got, strict=True)):
+            assert a.dtype == b.dtype and same_bits(a, b), (total, i)
 
 
 def test_a_longer_queue_costs_its_share():
