@@ -690,9 +690,9 @@ __global__ void __launch_bounds__(128, 4) server_kernel(const __grid_constant__ 
     }
 }
 
-// The lanes a world, from the worlds, their queues' slots and their rows: one when there are worlds enough to keep the chip's
-// warps in flight a thread each (a thread's accesses then coalesce with its neighbours', where a group's lanes read a slot
-// each, a sector or two apart for every world), else enough for the slots and rows at once, up to a warp (a larger queue or
+// The lanes a world, from the worlds, their queues' slots and their rows: one when there are worlds enough to keep the
+// chip's warps in flight a thread each (a thread's accesses then coalesce with its neighbours', where a group's lanes read
+// a slot each, a sector or two apart for every world), else enough for the slots and rows at once, up to a warp (a larger queue or
 // world is taken 32 at a time). A lane a world is a chain over its slots and rows, which takes as long for one world as for
 // thousands; groups take the longer the more warps they fill: so the line rises with the rows, and with the rounds of a
 // queue longer than a warp. It lies where the two cost the same (a server tick with its park's, us, one lane and a group):
