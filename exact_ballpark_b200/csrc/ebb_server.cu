@@ -692,14 +692,14 @@ __global__ void __launch_bounds__(128, 4) server_kernel(const __grid_constant__ 
 
 // The lanes a world, from the worlds, their queues' slots and their rows: one when there are worlds enough to keep the
 // chip's warps in flight a thread each (a thread's accesses then coalesce with its neighbours', where a group's lanes read
-// a slot each, a sector or two apart for every world), else enough for the slots and rows at once, up to a warp (a larger queue or
-// world is taken 32 at a time). A lane a world is a chain over its slots and rows, which takes as long for one world as for
-// thousands; groups take the longer the more warps they fill: so the line rises with the rows, and with the rounds of a
-// queue longer than a warp. It lies where the two cost the same (a server tick with its park's, us, one lane and a group):
-// rows, slots 2, 16: 4,096 worlds 45 and 41, 6,144 43 and 63; 4, 8: 12,288 29 and 24, 24,576 37 and 38; 5, 10: 4,096 37 and
-// 34, 8,192 37 and 48, 65,536 88 and 298; 16, 16: 12,288 87 and 84, 24,576 135 and 173; 4, 32: 2,048 78 and 54, 4,096 80 and
-// 89, 65,536 199 and 1,181; 9, 18: 3,072 62 and 53, 4,096 64 and 72; 32, 4: 8,192 85 and 70, 16,384 114 and 143; 32, 64:
-// 32,768 499 and 471, 49,152 587 and 709; 128, 256: 16,384 1,741 and 876.
+// a slot each, a sector or two apart for every world), else enough for the slots and rows at once, up to a warp (a larger
+// queue or world is taken 32 at a time). A lane a world is a chain over its slots and rows, which takes as long for one
+// world as for thousands; groups take the longer the more warps they fill: so the line rises with the rows, and with the
+// rounds of a queue longer than a warp. It lies about where the two cost the same (a server tick with its park's, us, one
+// lane and a group): rows, slots 2, 16: 4,096 worlds 45 and 41, 6,144 43 and 63; 4, 8: 12,288 29 and 24, 24,576 37 and 38;
+// 5, 10: 4,096 37 and 34, 8,192 37 and 48, 65,536 88 and 298; 16, 16: 12,288 87 and 84, 24,576 135 and 173; 4, 32: 2,048 78
+// and 54, 4,096 80 and 89, 65,536 199 and 1,181; 9, 18: 3,072 62 and 53, 4,096 64 and 72; 32, 4: 8,192 85 and 70, 16,384 114
+// and 143; 32, 64: 32,768 499 and 471, 49,152 587 and 709; 128, 256: 16,384 1,741 and 876.
 enum class Lanes { one, four, eight, half, warp };
 inline Lanes lanes(int64_t worlds, int64_t slots, int64_t width) {
     const int64_t most = slots > width ? slots : width, rows = width < 4096 ? width : 4096;
