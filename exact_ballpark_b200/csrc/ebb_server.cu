@@ -22,6 +22,8 @@
 // rounding pinned as in the flight tick (doubles by __dadd_rn and friends, the setters' float arguments rounded to
 // float, the rotation in float).
 
+#include <algorithm>
+
 #include "../../include/ebb.h"
 #include "ebb_flight.cuh"
 #include "ebb_rows.cuh"
@@ -698,15 +700,17 @@ __global__ void __launch_bounds__(128, 4) server_kernel(const __grid_constant__ 
 // rounds of a queue longer than a warp. It lies about where the two cost the same (a server tick with its park's, us, one
 // lane and a group): rows, slots 2, 16: 4,096 worlds 45 and 41, 6,144 43 and 63; 4, 8: 12,288 29 and 24, 24,576 37 and 38;
 // 5, 10: 4,096 37 and 34, 8,192 37 and 48, 65,536 88 and 298; 16, 16: 12,288 87 and 84, 24,576 135 and 173; 4, 32: 2,048 78
-// and 54, 4,096 80 and 89, 65,536 199 and 1,181; 9, 18: 3,072 62 and 53, 4,096 64 and 72; 32, 4: 8,192 85 and 70, 16,384 114
-// and 143; 32, 64: 32,768 499 and 471, 49,152 587 and 709; 128, 256: 16,384 1,741 and 876.
+// and 54, 4,096 80 and 89, 65,536 199 and 1,181; 9, 18: 3,072 62 and 53, 4,096 64 and 72; 16, 32: 4,096 106 and 78, 8,192
+// 124 and 128, 16,384 158 and 275; 32, 4: 8,192 85 and 70, 16,384 114 and 143; 32, 64: 32,768 499 and 471, 49,152 587 and
+// 709; 128, 256: 16,384 1,741 and 876.
 enum class Lanes { one, four, eight, half, warp };
 inline Lanes lanes(int64_t worlds, int64_t slots, int64_t width) {
     const int64_t most = slots > width ? slots : width, rows = width < 4096 ? width : 4096;
-    const int64_t line = most <= 8    ? 2048 * most
-                         : most <= 16 ? 4096 + 32 * rows * rows
-                         : slots <= 32 ? 2048 + 224 * rows
-                                       : (2048 + 224 * rows) * (64 + slots) / 32;
+    const int64_t chain = 2048 + 224 * rows, full = std::min<int64_t>(36 * rows * rows, 6144 + 128 * rows);
+    const int64_t line = most <= 8     ? 2048 * most
+                         : most <= 16  ? 4096 + 32 * rows * rows
+                         : slots <= 32 ? std::max(chain, full)
+                                       : chain * (64 + slots) / 32;
     if (worlds > line) return Lanes::one;
     return most <= 4 ? Lanes::four : most <= 8 ? Lanes::eight : most <= 16 ? Lanes::half : Lanes::warp;
 }
