@@ -366,7 +366,7 @@ __device__ bool ids_in_order(const World& x, const Group<G>& g, int64_t* span_ou
 constexpr int IDS_IN_REGISTERS = 8;
 
 template <bool WIDE>
-__device__ void queue_alone(const World& x, const EbbServerQueue& q) {
+__device__ __forceinline__ void queue_alone(const World& x, const EbbServerQueue& q) {
     const EbbServerState& s = x.s;
     const int64_t W = s.worlds, w = x.w, J = q.slots;
     const int32_t* __restrict__ kinds = q.kinds;
@@ -439,13 +439,6 @@ __device__ void queue_alone(const World& x, const EbbServerQueue& q) {
         trows_out[a] = trow;
         locs_out[a] = loc;
     }
-}
-
-__device__ void queue_alone(const World& x, const EbbServerQueue& q) {
-    if (x.s.width <= IDS_IN_REGISTERS)
-        queue_alone<false>(x, q);
-    else
-        queue_alone<true>(x, q);
 }
 
 // The queue pass: each push's rows, CloakBall's bubble and the duplicate test; nothing written to the park. Returns whether
@@ -527,8 +520,8 @@ __device__ void apply_slot(const World& x, const EbbServerQueue& q, int64_t j) {
     x.apply(kind, row, q.trow[a], f, q.n[a]);
 }
 
-template <int G>
-__device__ void queue_and_apply(const World& x, const EbbServerQueue& q, const Group<G>& g) {
+template <int G, bool WIDE>
+__device__ __forceinline__ void queue_and_apply(const World& x, const EbbServerQueue& q, const Group<G>& g) {
     const EbbServerState& s = x.s;
     const int64_t W = s.worlds, w = x.w;
     const int64_t clock = g.on ? x.p.clock[x.rows[0]] : 0;
@@ -539,7 +532,7 @@ __device__ void queue_and_apply(const World& x, const EbbServerQueue& q, const G
     }
     bool serial = true;                                   // (a world's only lane walks its queue)
     if constexpr (G == 1) {
-        if (g.on) queue_alone(x, q);
+        if (g.on) queue_alone<WIDE>(x, q);
     } else {
         serial = queue(x, q, g);
     }
@@ -660,8 +653,9 @@ __device__ void flags(const World& x, const EbbServerQueue& q, const Group<G>& g
 }
 
 // (4 blocks a multiprocessor, 128 registers: latency-bound; a lane a world of 65,536 takes 24.7 us so, 30.7 us at 5 blocks,
-// 40.1 at 6)
-template <int G>
+// 40.1 at 6. WIDE, a lane a world of more than IDS_IN_REGISTERS rows, is a kernel of its own: in one with the narrow worlds'
+// these, 65,536 of 4 ships, took 70 us a tick with the park's in place of 68; with the queue pass out of line 71.)
+template <int G, bool WIDE = false>
 __global__ void __launch_bounds__(128, 4) server_kernel(const __grid_constant__ EbbServerState s,
                                                       const __grid_constant__ EbbServerQueue q, int phase, int64_t j0,
                                                       int64_t j1) {
@@ -671,15 +665,15 @@ __global__ void __launch_bounds__(128, 4) server_kernel(const __grid_constant__ 
     switch (phase) {
         case 0:
         case 5:                                           // 5: phase 0, then the park's tick's dead-bubble test
-            queue_and_apply(x, q, g);
+            queue_and_apply<G, WIDE>(x, q, g);
             history(x, q, g, 0, q.slots);
             break;
-        case 1: queue_and_apply(x, q, g); break;
+        case 1: queue_and_apply<G, WIDE>(x, q, g); break;
         case 2: history(x, q, g, j0, j1); break;
         case 3: flags(x, q, g); break;
         case 6:                                           // the queue's test alone: flags, rows, CloakBall's bubble
             if constexpr (G == 1) {
-                if (g.on) queue_alone(x, q);
+                if (g.on) queue_alone<WIDE>(x, q);
             } else {
                 queue(x, q, g);
             }
@@ -714,11 +708,11 @@ inline Lanes lanes(int64_t worlds, int64_t slots, int64_t width) {
     if (worlds > line) return Lanes::one;
     return most <= 4 ? Lanes::four : most <= 8 ? Lanes::eight : most <= 16 ? Lanes::half : Lanes::warp;
 }
-template <int G>
+template <int G, bool WIDE = false>
 cudaError_t launch(const EbbServerState& s, const EbbServerQueue& q, int phase, int64_t j0, int64_t j1, cudaStream_t st,
                    int block) {
     const unsigned grid = (unsigned)((s.worlds + block / G - 1) / (block / G));
-    server_kernel<G><<<grid, block, 0, st>>>(s, q, phase, j0, j1);
+    server_kernel<G, WIDE><<<grid, block, 0, st>>>(s, q, phase, j0, j1);
     return cudaGetLastError();
 }
 
@@ -751,11 +745,14 @@ int ebb_server_tick(const EbbServerState* s, const EbbServerQueue* q, int phase,
         return EBB_EINVAL;
     const cudaStream_t st = (cudaStream_t)stream;
     const ebb::server::Lanes g = ebb::server::lanes(s->worlds, q->slots, s->width);
-    const cudaError_t e = g == ebb::server::Lanes::one     ? ebb::server::launch<1>(*s, *q, phase, j0, j1, st, block)
-                          : g == ebb::server::Lanes::four  ? ebb::server::launch<4>(*s, *q, phase, j0, j1, st, block)
-                          : g == ebb::server::Lanes::eight ? ebb::server::launch<8>(*s, *q, phase, j0, j1, st, block)
-                          : g == ebb::server::Lanes::half  ? ebb::server::launch<16>(*s, *q, phase, j0, j1, st, block)
-                                                           : ebb::server::launch<32>(*s, *q, phase, j0, j1, st, block);
+    const bool wide = s->width > ebb::server::IDS_IN_REGISTERS;
+    const cudaError_t e =
+        g == ebb::server::Lanes::one     ? (wide ? ebb::server::launch<1, true>(*s, *q, phase, j0, j1, st, block)
+                                                 : ebb::server::launch<1>(*s, *q, phase, j0, j1, st, block))
+        : g == ebb::server::Lanes::four  ? ebb::server::launch<4>(*s, *q, phase, j0, j1, st, block)
+        : g == ebb::server::Lanes::eight ? ebb::server::launch<8>(*s, *q, phase, j0, j1, st, block)
+        : g == ebb::server::Lanes::half  ? ebb::server::launch<16>(*s, *q, phase, j0, j1, st, block)
+                                         : ebb::server::launch<32>(*s, *q, phase, j0, j1, st, block);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
